@@ -83,9 +83,7 @@ __device__ __forceinline__ bool tile_ticket_last(unsigned *ticket, int ntiles)
 
 __device__ __forceinline__ double tile_partials_sum(const double *p, int n, double *sm)
 {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < n; b += blockDim.x) s += ((volatile const double *)p)[b];
-    return block_sum(s, sm);
+    return partials_sum(p, n, sm);
 }
 
 // site of step s of this thread in tile `tile` (a tile is spt x BS consecutive sites)
@@ -105,7 +103,7 @@ __device__ __forceinline__ unsigned group_mask(const GroupDesc &G)
     for (int r = 0; r < R; ++r)
         if (r < G.n) {
             const MsState *st = c_sys[G.mem[r]].st;
-            if (st->active && st->mode == M) use |= 1u << r;
+            if (st->active[0] && st->mode == M) use |= 1u << r;
         }
     return use;
 }
@@ -250,14 +248,14 @@ __global__ void __launch_bounds__(BS) bk_init_kernel(const int2 *__restrict__ it
                 }
                 st->maxTerm = st->ns;
                 st->wmax = st->ns;
-                st->iter = st->wpos = st->nupd = st->halt = 0;
+                st->iter = st->wpos = st->halt = 0;
                 st->mode = st->next_mode = 0;
                 st->pp = tot;  // p0 = b
                 // b = 0: x = 0 is the solution; a non-finite source is a breakdown
                 const bool finite = isfinite(tot);
                 st->status = finite ? 0 : KQ_STATUS_BREAKDOWN;
-                st->active = (finite && tot > 0.0) ? 1 : 0;
-                if (!st->active && st->running) atomicSub(st->running, 1);
+                st->active[0] = (finite && tot > 0.0) ? 1 : 0;
+                if (!st->active[0] && st->running) atomicSub(st->running, 1);
                 st->ticket[0] = 0;
             }
         }
@@ -327,9 +325,9 @@ __global__ void __launch_bounds__(BS, Bounds<BS, M, Pass<M, R, P64>::v>::v) bk_d
                 if (threadIdx.x == 0) d.partials[w.y] = bt;
                 if (tile_ticket_last(&st->ticket[1], d.ntiles)) {
                     const double tot = tile_partials_sum(d.partials, d.ntiles, sm);
-                    if (threadIdx.x < 32) {
-                        ms_step_beta(st, st->shift[0] * st->pp + __shfl_sync(0xffffffffu, tot, 0));
-                        if (threadIdx.x == 0) st->ticket[1] = 0;
+                    if (threadIdx.x == 0) {
+                        ms_beta(st, 0, st->rNorm2, st->shift[0] * st->pp + tot);
+                        st->ticket[1] = 0;
                     }
                 }
                 __syncthreads();
@@ -379,7 +377,7 @@ __global__ void __launch_bounds__(BS, Bounds<BS, M, Pass<M, R, P64>::v>::v) bk_d
                         double pv6[6], rv[6];
                         ld_spinor<0>(d.p0, d.pv, i, pv6);
                         ld_spinor<0>(rin, d.pv, i, rv);
-                        const double sig = st->shift[0], b0 = st->B[0];
+                        const double sig = st->shift[0], b0 = st->b0;
 #pragma unroll
                         for (int k = 0; k < 6; ++k) {
                             rv[k] += b0 * (sig * pv6[k] - (double)acc[r][k]);
@@ -398,9 +396,9 @@ __global__ void __launch_bounds__(BS, Bounds<BS, M, Pass<M, R, P64>::v>::v) bk_d
                 if (threadIdx.x == 0) d.partials[w.y] = bn;
                 if (tile_ticket_last(&st->ticket[2], d.ntiles)) {
                     const double tot = tile_partials_sum(d.partials, d.ntiles, sm);
-                    if (threadIdx.x < 32) {
-                        ms_step_alpha(st, __shfl_sync(0xffffffffu, tot, 0));
-                        if (threadIdx.x == 0) st->ticket[2] = 0;
+                    if (threadIdx.x == 0) {
+                        ms_alpha(st, st->rNorm2, tot);
+                        st->ticket[2] = 0;
                     }
                 }
                 __syncthreads();
@@ -597,9 +595,9 @@ __device__ __forceinline__ void staged_member_steps(const GroupDesc &G, unsigned
             }
             if (tile_ticket_last(&st->ticket[ticket], d.ntiles)) {
                 const double tot = tile_partials_sum(d.partials, d.ntiles, sm);
-                if (threadIdx.x < 32) {
-                    step(st, __shfl_sync(0xffffffffu, tot, 0));
-                    if (threadIdx.x == 0) st->ticket[ticket] = 0;
+                if (threadIdx.x == 0) {
+                    step(st, tot);
+                    st->ticket[ticket] = 0;
                 }
             }
             __syncthreads();
@@ -646,7 +644,7 @@ __global__ void __launch_bounds__(BS, Bounds<BS, M, 1>::v) bk_dslash1_staged_ker
                                        for (int k = 0; k < 6; ++k) tt += (double)acc[k] * (double)acc[k];
                                    });
         staged_member_steps<BS, R>(G, use, w.y, tt, 1, wsum, sm, [](MsState *st, double tot) {
-            ms_step_beta(st, st->shift[0] * st->pp + tot);
+            ms_beta(st, 0, st->rNorm2, st->shift[0] * st->pp + tot);
         });
     }
 }
@@ -686,7 +684,7 @@ __global__ void __launch_bounds__(BS, Bounds<BS, M, 1>::v) bk_dslash2_staged_ker
                                        double pv6[6], rv[6];
                                        ld_spinor<0>(d.p0, d.pv, i, pv6);
                                        ld_spinor<0>(rin, d.pv, i, rv);
-                                       const double sig = st->shift[0], b0 = st->B[0];
+                                       const double sig = st->shift[0], b0 = st->b0;
 #pragma unroll
                                        for (int k = 0; k < 6; ++k) {
                                            rv[k] += b0 * (sig * pv6[k] - (double)acc[k]);
@@ -695,12 +693,12 @@ __global__ void __launch_bounds__(BS, Bounds<BS, M, 1>::v) bk_dslash2_staged_ker
                                        st_spinor<0>(rout, d.pv, i, rv);
                                    });
         staged_member_steps<BS, R>(G, use, w.y, nn, 2, wsum, sm,
-                                   [](MsState *st, double tot) { ms_step_alpha(st, tot); });
+                                   [](MsState *st, double tot) { ms_alpha(st, st->rNorm2, tot); });
     }
 }
 
-// K3: p0 = r^(i) + a0 p0 (and its copy in the next iteration's precision when that is FP32 or HALF); the next
-// iteration's precision takes effect.  A system that stopped in K2 no longer needs p0.
+// K3: p0 = r^(i) + a0 p0 (and its copy in the next iteration's precision when that is FP32 or HALF); the system's
+// last tile takes the shift step, and the next iteration's precision takes effect.
 template <int BS>
 __global__ void __launch_bounds__(BS) bk_p0_kernel(const int2 *__restrict__ items, int nitems, int spt)
 {
@@ -709,9 +707,9 @@ __global__ void __launch_bounds__(BS) bk_p0_kernel(const int2 *__restrict__ item
         const int2 w = items[it];
         const SysDesc &d = c_sys[w.x];
         MsState *st = d.st;
-        if (!st->active) continue;
+        if (!st->active[0]) continue;
         const char *r = static_cast<const char *>(d.ring) + (size_t)(st->iter % kWin) * d.vb;
-        const double a0 = st->a[0];
+        const double a0 = st->a0;
         const int nm = st->next_mode;  // the next iteration's operator precision (set by the alpha step)
         for (int sidx = 0; sidx < spt; ++sidx) {
             const int i = tile_site<BS>(w.y, spt, sidx);
@@ -726,9 +724,16 @@ __global__ void __launch_bounds__(BS) bk_p0_kernel(const int2 *__restrict__ item
             if (nm == 1) st_spinor_as<1>(d.p0s, d.pv, i, pv6);
             else if (nm == 2) st_spinor_as<2>(d.p0s, d.pv, i, pv6);
         }
-        if (tile_ticket_last(&st->ticket[3], d.ntiles) && threadIdx.x == 0) {
-            st->mode = st->next_mode;
-            st->ticket[3] = 0;
+        if (tile_ticket_last(&st->ticket[3], d.ntiles)) {
+            const bool go = ms_shift_step(st);
+            if (threadIdx.x == 0) {
+                if (!go) {
+                    st->active[0] = 0;
+                    if (st->running) atomicSub(st->running, 1);
+                }
+                st->mode = st->next_mode;
+                st->ticket[3] = 0;
+            }
         }
         __syncthreads();
     }
@@ -746,7 +751,7 @@ __global__ void __launch_bounds__(BS) bk_window_kernel(const int2 *__restrict__ 
         MsState *st = d.st;
         const int n = st->wpos, kmax = st->wmax;
         // uniform per system: apply a full window, or a partial one once the system has stopped
-        if (n == 0 || (n < kWin && st->active)) continue;
+        if (n == 0 || (n < kWin && st->active[0])) continue;
         __syncthreads();
         for (int t = threadIdx.x; t < kmax; t += BS) {
             sc[t] = st->c[t];

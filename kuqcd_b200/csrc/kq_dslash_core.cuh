@@ -352,25 +352,50 @@ __device__ __forceinline__ double block_sum(double v, double *smem32)
     return v;  // valid in thread 0
 }
 
-// Publish this block's partial sum; returns true in the 32 threads of warp 0 of the last block to arrive, each
-// holding in *total the fixed-order sum of all partials.  Every block calls this unconditionally.
-__device__ __forceinline__ bool grid_sum_last_warp(double v, double *partials, unsigned *ticket, double *smem32,
-                                                   double *total)
+// Publish this block's partial sum; returns true in every thread of the last block to arrive.  Every block calls
+// this unconditionally.
+__device__ __forceinline__ bool grid_arrive(double v, double *partials, unsigned *ticket, double *smem32)
 {
     __shared__ bool am_last;
     v = block_sum(v, smem32);
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = v;
         __threadfence();
-        const unsigned t = atomicAdd(ticket, 1u);
-        am_last = (t == gridDim.x - 1);
+        am_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!am_last) return false;
     __threadfence();
+    return true;
+}
+
+// Fixed-order sum of n partials by the last block (the total in thread 0).  Each thread adds every blockDim.x-th
+// partial; eight loads are in flight before the first is added (one at a time, the 2048 partials of a 32^4 lattice
+// cost eight round trips to L2 in the tail of the kernel).
+__device__ __forceinline__ double partials_sum(const double *partials, int n, double *smem32)
+{
+    constexpr int U = 8;
     double s = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s += *((volatile double *)partials + b);
-    s = block_sum(s, smem32);
+    for (int b0 = threadIdx.x; b0 < n; b0 += U * blockDim.x) {
+        double w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int b = b0 + u * (int)blockDim.x;
+            w[u] = b < n ? __ldcg(partials + b) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) s += w[u];
+    }
+    return block_sum(s, smem32);
+}
+
+// grid_arrive + partials_sum: true in the 32 threads of warp 0 of the last block to arrive, each holding in *total
+// the fixed-order sum of all partials; the ticket is reset.
+__device__ __forceinline__ bool grid_sum_last_warp(double v, double *partials, unsigned *ticket, double *smem32,
+                                                   double *total)
+{
+    if (!grid_arrive(v, partials, ticket, smem32)) return false;
+    const double s = partials_sum(partials, (int)gridDim.x, smem32);
     if (threadIdx.x >= 32) return false;
     *total = __shfl_sync(0xffffffffu, s, 0);
     if (threadIdx.x == 0) *ticket = 0u;

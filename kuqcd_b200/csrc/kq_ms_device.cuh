@@ -2,141 +2,132 @@
 // and the batched multi-system solver (kq_batch.cu).  They restate the recurrences of inverter_cgm.cpp:45-77 and
 // accumulate the window coefficients of the deferred shift updates.
 #pragma once
+#include "kq_dslash_core.cuh"
 #include "kq_msrelax.h"
 
 namespace kq {
 
 // ---------------------------------------------------------------------------------------------------- scalar steps
-// Both steps are run by the 32 lanes of one warp (of the last block to finish the reduction).  Every lane reads the
-// shared scalars before any lane writes (__syncwarp); then lane l computes the per-shift scalars of shifts l and
-// l + 32, and after a __syncwarp the window coefficients are updated one (shift, position) item per lane.  Each
-// value has one writer per phase, so the result is that of the reference's sequential loops, while the loads of
-// different shifts overlap instead of forming a chain of dependent global-memory round trips (this runs in the
-// tail of a kernel, after every other block has finished).  The item loop keeps few values live, so the step does
-// not raise the register count of the dslash kernel that hosts it.
+// What the next kernel of the iteration waits for is taken at the end of each reduction by one thread: B_0 after the
+// first dslash (ms_beta), a_0 after the second (ms_alpha).  Everything else -- the shifted recurrences, the window
+// coefficients of the deferred updates, the dropping of converged shifts -- is one shift step per iteration, run by
+// a whole block beside the update of p0 (ms_shift_step).  With the shift work inside the two reductions, one warp
+// looping over (shift, position) items in global memory, the tail of either dslash kernel cost about 9 us: at 16^4
+// with 12 shifts the FP64 kernels took 23 us for 14 us of dslash.
 
-// beta step (inverter_cgm.cpp:48-57, 61-63): B_0 = -|r|^2 / <p, A p>, the shifted B_k and zeta_k, and
-// x_k -= B_k p_k in the window representation of p_k
-__device__ __forceinline__ void ms_step_beta(MsState *st, double pAp)
+// beta step (inverter_cgm.cpp:48-50): B_0 = -|r|^2 / <p, A p>, <p, A p> = sigma_0 |p|^2 + |D p|^2.  One thread;
+// `slot`: the flag of the running iteration.
+__device__ __forceinline__ void ms_beta(MsState *st, int slot, double rNorm2, double pAp)
 {
-    const int lane = threadIdx.x & 31;
-    const double rNorm2 = st->rNorm2, Bm1 = st->Bm1, a0 = st->a[0];
-    const int mt = st->maxTerm, ns = st->ns, jw = st->wpos;  // ring positions 0..jw-1 are in use
     const double B0 = -rNorm2 / pAp;
-    const bool bad = !(pAp != 0.0) || !isfinite(B0);
-    __syncwarp();
-    if (bad) {
-        if (lane == 0) {
-            st->pAp = pAp;
-            st->status = KQ_STATUS_BREAKDOWN;
-            st->active = 0;
-            st->halt = 1;
-        }
+    if (!(pAp != 0.0) || !isfinite(B0)) {
+        st->status = KQ_STATUS_BREAKDOWN;
+        st->active[slot] = 0;
+        st->halt = 1;
         return;
     }
-#pragma unroll 1
-    for (int k = lane; k < mt; k += 32) {
-        double Bk = B0;
-        if (k > 0) {
-            const double zm1 = st->Zm1[k], z = st->Z[k], sh = st->shift[k];
-            const double rr1 = Bm1 * zm1 / (B0 * a0 * (zm1 - z) + zm1 * Bm1 * (1.0 - sh * B0));
-            st->Zm1[k] = z;
-            st->Z[k] = z * rr1;
-            Bk = B0 * rr1;
-        }
-        st->B[k] = Bk;
-    }
-    __syncwarp();
-    if (jw == 0) {
-        // first iteration of a window: identity representation p = p_old (c = 1), x = x_old, then x -= B p
-#pragma unroll 1
-        for (int k = lane; k < ns; k += 32) {
-            st->c[k] = 1.0;
-            st->e[k] = k < mt ? -st->B[k] : 0.0;
-        }
-#pragma unroll 1
-        for (int t = lane; t < ns * kWin; t += 32) {
-            const int k = t / kWin, l = t - k * kWin;
-            st->d[k][l] = 0.0;
-            st->f[k][l] = 0.0;
-        }
-    } else {
-        // e_k -= B_k c_k (item l = jw) and f_kl -= B_k d_kl (items l < jw)
-        const int per = jw + 1;
-#pragma unroll 1
-        for (int t = lane; t < mt * per; t += 32) {
-            const int k = t / per, l = t - k * per;
-            const double Bk = st->B[k];
-            if (l == jw) st->e[k] -= Bk * st->c[k];
-            else st->f[k][l] -= Bk * st->d[k][l];
-        }
-    }
-    if (lane == 0) {
-        st->pAp = pAp;
-        st->Bm1 = B0;
-        st->nupd = mt;
-        if (jw == 0) st->wmax = mt;
-    }
+    st->b0 = B0;
 }
 
-// alpha step (inverter_cgm.cpp:58-60, 64-77): a_0 = |r_new|^2 / |r|^2, the shifted a_k, p_k = Z_k r_new + a_k p_k
-// in the window representation, and the converged shifts dropped from the top (zeta_k^2 |r|^2 < tol)
-__device__ __forceinline__ void ms_step_alpha(MsState *st, double lambda2)
+// alpha step (inverter_cgm.cpp:58-60): a_0 = |r_new|^2 / |r|^2, and the next iteration's operator precision (the
+// batched solver's).  One thread.
+__device__ __forceinline__ void ms_alpha(MsState *st, double rNorm2, double lambda2)
 {
-    const int lane = threadIdx.x & 31;
-    const double rNorm2 = st->rNorm2, B0 = st->B[0], tol = st->tol;
-    const int nu = st->nupd, jw = st->wpos, mt0 = st->maxTerm, halt0 = st->halt;
     const double a0 = lambda2 / rNorm2;
-    __syncwarp();
-    // a_k, and the new maxTerm: one above the highest shift still above tolerance (the reference's do-while)
-    int mt = 0;
-#pragma unroll
-    for (int base = 0; base < kMaxShift; base += 32) {
-        const int k = base + lane;
+    st->a0 = a0;
+    st->lambda2 = lambda2;
+    st->rNorm2 = lambda2;
+    // |p_new|^2 = |r_new|^2 + a0^2 |p|^2, since the step makes r_new orthogonal to p
+    st->pp = lambda2 + a0 * a0 * st->pp;
+    st->iter += 1;
+    if (!isfinite(lambda2)) {
+        st->status = KQ_STATUS_BREAKDOWN;
+        st->halt = 1;
+    }
+    const double rel2 = lambda2 / st->bnorm2;
+    st->next_mode = (st->rho16_2 > 0.0 && rel2 < st->rho16_2) ? 2 : (st->rho32_2 > 0.0 && rel2 < st->rho32_2) ? 1 : 0;
+}
+
+// Shift step of one iteration (inverter_cgm.cpp:51-57, 61-77), run by every thread of one block of at least 64
+// threads after ms_alpha: thread k < 64 takes shift k's recurrences (the shifted B_k, zeta_k, a_k, and whether the
+// shift is still above tolerance), then the (shift, position) items of the window coefficients are spread over the
+// block.  x_k -= B_k p_k and p_k = Z_k r_new + a_k p_k in the window representation are
+//     e_k -= B_k c_k, f_kl -= B_k d_kl, then c_k *= a_k, d_kl *= a_k, d_k,new = Z_k.
+// Every value is loaded once, all loads of a phase are independent, and each value has one writer.  Returns (to every
+// thread) whether the solve goes on.
+__device__ __forceinline__ bool ms_shift_step(MsState *st)
+{
+    __shared__ double sB[kMaxShift], sa[kMaxShift], sZ[kMaxShift];
+    __shared__ unsigned keep_mask[kMaxShift / 32];
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int mt0 = st->maxTerm, ns = st->ns, jw = st->wpos;  // ring positions 0..jw-1 are in use
+    const double B0 = st->b0, a0 = st->a0, a0m1 = st->a[0], Bm1 = st->Bm1, lambda2 = st->lambda2, tol = st->tol;
+    if (tid < kMaxShift) {
+        const int k = tid;
+        double Bk = B0, ak = a0, z = 1.0;
         bool keep = false;
-        if (k < nu) st->a[k] = k == 0 ? a0 : a0 * st->Z[k] * st->B[k] / (st->Zm1[k] * B0);
         if (k < mt0) {
-            const double z = st->Z[k];
-            keep = !(z * z * lambda2 < tol);
+            z = st->Z[k];
+            if (k > 0) {
+                const double zm1 = st->Zm1[k], sh = st->shift[k];
+                const double rr1 = Bm1 * zm1 / (B0 * a0m1 * (zm1 - z) + zm1 * Bm1 * (1.0 - sh * B0));
+                const double zn = z * rr1;
+                Bk = B0 * rr1;
+                ak = a0 * zn * Bk / (z * B0);
+                st->Zm1[k] = z;
+                st->Z[k] = zn;
+                z = zn;
+            }
+            st->B[k] = Bk;
+            keep = !(z * z * lambda2 < tol);  // converged shifts drop from the top
+            sB[k] = Bk;
+            sa[k] = ak;
+            sZ[k] = z;
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (m) mt = base + 32 - __clz((int)m);
+        if ((tid & 31) == 0) keep_mask[tid >> 5] = m;
     }
-    __syncwarp();
-    // c_k *= a_k (item l = jw, which also records Z_k as the weight of the new residual), d_kl *= a_k (l < jw)
-    const int per = jw + 1;
-#pragma unroll 1
-    for (int t = lane; t < nu * per; t += 32) {
-        const int k = t / per, l = t - k * per;
-        const double ak = st->a[k];
-        if (l == jw) {
-            st->c[k] *= ak;
-            st->d[k][jw] = st->Z[k];
-        } else {
-            st->d[k][l] *= ak;
+    __syncthreads();
+    if (tid < mt0) st->a[tid] = sa[tid];
+    // the new maxTerm: one above the highest shift still above tolerance (the reference's do-while)
+    int mt = 0;
+#pragma unroll
+    for (int w = 0; w < kMaxShift / 32; ++w)
+        if (keep_mask[w]) mt = 32 * (w + 1) - __clz((int)keep_mask[w]);
+    if (jw == 0) {
+        // first iteration of a window: from the identity representation p = p_old, x = x_old
+        for (int t = tid; t < ns * kWin; t += nt) {
+            const int k = t / kWin, l = t - k * kWin;
+            const bool on = k < mt0;
+            st->d[k][l] = on && l == 0 ? sZ[k] : 0.0;
+            st->f[k][l] = 0.0;
+            if (l == 0) {
+                st->c[k] = on ? sa[k] : 1.0;
+                st->e[k] = on ? -sB[k] : 0.0;
+            }
+        }
+    } else {
+        // item l = jw: c_k, e_k and the weight of the new residual; items l < jw: d_kl, f_kl
+        const int per = jw + 1;
+#pragma unroll 4
+        for (int t = tid; t < mt0 * per; t += nt) {
+            const int k = t / per, l = t - k * per;
+            double *dp = l == jw ? &st->c[k] : &st->d[k][l], *fp = l == jw ? &st->e[k] : &st->f[k][l];
+            const double dv = *dp, fv = *fp;
+            *fp = fv - sB[k] * dv;
+            *dp = dv * sa[k];
+            if (l == jw) st->d[k][jw] = sZ[k];
         }
     }
-    if (lane == 0) {
-        st->lambda2 = lambda2;
-        st->a[0] = a0;
-        st->rNorm2 = lambda2;
-        // |p_new|^2 = |r_new|^2 + a0^2 |p|^2, since the step makes r_new orthogonal to p
-        st->pp = lambda2 + a0 * a0 * st->pp;
+    const bool go = mt > 0 && st->iter < st->max_iter && !st->halt && isfinite(lambda2);
+    __syncthreads();  // every thread has read what thread 0 overwrites
+    if (tid == 0) {
         st->maxTerm = mt;
-        st->iter += 1;
+        st->Bm1 = B0;
         st->wpos = jw + 1;
-        const bool finite = isfinite(lambda2);
-        if (!finite) {
-            st->status = KQ_STATUS_BREAKDOWN;
-            st->halt = 1;
-        }
-        st->active = (mt > 0 && st->iter < st->max_iter && !halt0 && finite) ? 1 : 0;
-        if (!st->active && st->running) atomicSub(st->running, 1);
-        // relaxed operator precision for the next iteration, from the base residual (the batched solver's)
-        const double rel2 = lambda2 / st->bnorm2;
-        st->next_mode =
-            (st->rho16_2 > 0.0 && rel2 < st->rho16_2) ? 2 : (st->rho32_2 > 0.0 && rel2 < st->rho32_2) ? 1 : 0;
+        if (jw == 0) st->wmax = mt0;
     }
+    return go;
 }
 
 // Windowed shift update of one site, one colour component at a time (keeps W ring values in registers, not 6 W):

@@ -23,9 +23,9 @@
 //    with a 16-bit temporary the step length uses |D p|^2 before the temporary is rounded (relative 3e-5), while
 //    the residual update uses the operator actually applied, so the recurrence stays exact.
 //
-// Kernels per iteration: K1 tmp = D p0, |tmp|^2 (beta step + x coefficients);  K2 r <- r + B0 (sigma0 p0 - D tmp)
-// into the ring, |r|^2 (alpha step + p coefficients + shift dropping + |p0|^2 = |r|^2 + a0^2 |p0|^2, r being
-// orthogonal to the old p0);  K3 p0 <- r + a0 p0.
+// Kernels per iteration: K1 tmp = D p0, |tmp|^2 (beta step);  K2 r <- r + B0 (sigma0 p0 - D tmp) into the ring,
+// |r|^2 (alpha step + |p0|^2 = |r|^2 + a0^2 |p0|^2, r being orthogonal to the old p0);  K3 p0 <- r + a0 p0, with the
+// shift step (shifted recurrences, window coefficients, shift dropping) in one block of its own beside it.
 // One CUDA graph per operator precision, kChunk iterations each followed by K4, the windowed shift update, which
 // applies the window once it is full (W = 2 kChunk iterations) or the solve has stopped, and otherwise returns at
 // once.  The window sets the shift-update traffic, the chunk the granularity of the precision switches.
@@ -80,23 +80,24 @@ __global__ void __launch_bounds__(kBSm) ms_init_kernel(int vh, int pv, const voi
         st->wmax = st->ns;
         st->iter = 0;
         st->wpos = 0;
-        st->nupd = 0;
         st->halt = 0;
         // b = 0: x = 0 is the solution; a non-finite source is a breakdown
         const bool finite = isfinite(tot);
         st->status = finite ? 0 : KQ_STATUS_BREAKDOWN;
-        st->active = (finite && tot > 0.0) ? 1 : 0;
+        st->active[0] = (finite && tot > 0.0) ? 1 : 0;
+        st->active[1] = 0;
     }
 }
 
 // K1: tmp = D p0 (p0 FP64; links LP; tmp stored in SO); |tmp|^2, then the beta step with
-// <p0, A p0> = sigma0 |p0|^2 + |tmp|^2 (|p0|^2 from the alpha step's recurrence)
+// <p0, A p0> = sigma0 |p0|^2 + |tmp|^2 (|p0|^2 from the alpha step's recurrence).  slot: parity of the iteration
+// within its chunk.
 template <int LP, int SO>
 __global__ void __launch_bounds__(kBSm) ms_dslash1_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
                                                           const void *__restrict__ p0, void *__restrict__ tmp, int q,
-                                                          MsState *st, double *partials)
+                                                          int slot, MsState *st, double *partials)
 {
-    if (st->active == 0) return;
+    if (st->active[slot] == 0) return;
     __shared__ double sm[32];
     const int i = blockIdx.x * kBSm + threadIdx.x;
     double tt = 0.0;
@@ -108,8 +109,13 @@ __global__ void __launch_bounds__(kBSm) ms_dslash1_kernel(Geom g, int pv, LinkSe
 #pragma unroll
         for (int k = 0; k < 6; ++k) tt += (double)acc[k] * (double)acc[k];
     }
-    double tot;
-    if (grid_sum_last_warp(tt, partials, &st->ticket[1], sm, &tot)) ms_step_beta(st, st->shift[0] * st->pp + tot);
+    if (!grid_arrive(tt, partials, &st->ticket[1], sm)) return;
+    const double sp = st->shift[0] * st->pp, rr = st->rNorm2;  // in flight with the partials
+    const double tot = partials_sum(partials, (int)gridDim.x, sm);
+    if (threadIdx.x == 0) {
+        st->ticket[1] = 0u;
+        ms_beta(st, slot, rr, sp + tot);
+    }
 }
 
 // K2: s = sigma0 p0 - D tmp (tmp stored in SI, links LP; s stays in registers); r^(i+1) = r^(i) + B0 s into the
@@ -117,10 +123,10 @@ __global__ void __launch_bounds__(kBSm) ms_dslash1_kernel(Geom g, int pv, LinkSe
 template <int LP, int SI>
 __global__ void __launch_bounds__(kBSm) ms_dslash2_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
                                                           const void *__restrict__ tmp, const void *__restrict__ p0,
-                                                          char *ring, size_t vb, int p, MsState *st,
-                                                          double *partials)
+                                                          char *ring, size_t vb, int p, int slot,
+                                                          MsState *st, double *partials)
 {
-    if (st->active == 0) return;
+    if (st->active[slot] == 0) return;
     __shared__ double sm[32];
     const int it = st->iter;  // iterations completed before this one
     const char *rin = ring + (size_t)(it % kWin) * vb;
@@ -134,7 +140,7 @@ __global__ void __launch_bounds__(kBSm) ms_dslash2_kernel(Geom g, int pv, LinkSe
         double pv6[6], rv[6];
         ld_spinor<0>(p0, pv, i, pv6);
         ld_spinor<0>(rin, pv, i, rv);
-        const double sig = st->shift[0], b0 = st->B[0];
+        const double sig = st->shift[0], b0 = st->b0;
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
             rv[k] += b0 * (sig * pv6[k] - (double)acc[k]);
@@ -142,22 +148,33 @@ __global__ void __launch_bounds__(kBSm) ms_dslash2_kernel(Geom g, int pv, LinkSe
         }
         st_spinor<0>(rout, pv, i, rv);
     }
-    double tot;
-    if (grid_sum_last_warp(nn, partials, &st->ticket[2], sm, &tot)) ms_step_alpha(st, tot);
+    if (!grid_arrive(nn, partials, &st->ticket[2], sm)) return;
+    const double rr = st->rNorm2;
+    const double tot = partials_sum(partials, (int)gridDim.x, sm);
+    if (threadIdx.x == 0) {
+        st->ticket[2] = 0u;
+        ms_alpha(st, rr, tot);
+    }
 }
 
-// K3: p0 = r^(i) + a0 p0
+// K3: p0 = r^(i) + a0 p0; block 0 takes the shift step meanwhile
 __global__ void __launch_bounds__(kBSm) ms_p0_kernel(int vh, int pv, const char *ring, size_t vb, void *p0,
-                                                     const MsState *st)
+                                                     int slot, MsState *st)
 {
-    if (st->active == 0) return;
-    const int i = blockIdx.x * kBSm + threadIdx.x;
+    const bool on = st->active[slot] != 0;
+    if (blockIdx.x == 0) {
+        const bool go = on && ms_shift_step(st);
+        if (threadIdx.x == 0) st->active[1 - slot] = go ? 1 : 0;
+        return;
+    }
+    if (!on) return;
+    const int i = (blockIdx.x - 1) * kBSm + threadIdx.x;
     if (i >= vh) return;
     const char *r = ring + (size_t)(st->iter % kWin) * vb;
     double rv[6], pv6[6];
     ld_spinor<0>(r, pv, i, rv);
     ld_spinor<0>(p0, pv, i, pv6);
-    const double a0 = st->a[0];
+    const double a0 = st->a0;
 #pragma unroll
     for (int k = 0; k < 6; ++k) pv6[k] = rv[k] + a0 * pv6[k];
     st_spinor<0>(p0, pv, i, pv6);
@@ -173,7 +190,7 @@ __global__ void __launch_bounds__(kBSm, 2) ms_window_kernel(int vh, int pv, cons
     if (threadIdx.x == 0) {
         nw = st->wpos;
         km = st->wmax;
-        act = st->active;
+        act = st->active[0];
     }
     __syncthreads();
     const int n = nw, kmax = km;
@@ -221,11 +238,11 @@ static void enqueue_ms_chunk(const Geom &g, const GaugeDev &gd, const MsBuffers 
 {
     const int pv = pad_sites(g.vh), nb = (g.vh + kBSm - 1) / kBSm;
     for (int it = 0; it < kChunk; ++it) {
-        ms_dslash1_kernel<LP, SO><<<nb, kBSm, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.p0, w.tmp, 1 - parity, w.st,
+        ms_dslash1_kernel<LP, SO><<<nb, kBSm, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.p0, w.tmp, 1 - parity, it & 1, w.st,
                                                       w.partials);
         ms_dslash2_kernel<LP, SO><<<nb, kBSm, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.tmp, w.p0, (char *)w.ring,
-                                                      w.vb, parity, w.st, w.partials);
-        ms_p0_kernel<<<nb, kBSm, 0, s>>>(g.vh, pv, (const char *)w.ring, w.vb, w.p0, w.st);
+                                                      w.vb, parity, it & 1, w.st, w.partials);
+        ms_p0_kernel<<<nb + 1, kBSm, 0, s>>>(g.vh, pv, (const char *)w.ring, w.vb, w.p0, it & 1, w.st);
     }
     switch (window_unroll()) {
         case 1: ms_window_kernel<1><<<nb, kBSm, 0, s>>>(g.vh, pv, (const char *)w.ring, w.vb, (char *)w.pw, (char *)w.x, w.st); break;
@@ -318,7 +335,7 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
         err = cudaMemcpyAsync(poll, w.st, sizeof(MsPoll), cudaMemcpyDeviceToHost, s);
         if (err == cudaSuccess) err = cudaStreamSynchronize(s);
         if (err != cudaSuccess) break;
-        if (!poll->active) {
+        if (!poll->active[0]) {
             if (poll->wpos == 0) report(0);  // stopped, last window flushed: every x_k is final
             break;
         }

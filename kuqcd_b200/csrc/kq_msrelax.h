@@ -6,18 +6,23 @@ namespace kq {
 
 constexpr int kWin = 16;   // iterations per shift-update window (ring of residuals)
 constexpr int kChunk = 8;  // iterations per CUDA graph: the host picks the operator precision between chunks
+static_assert(kChunk % 2 == 0, "a chunk starts on active[0]");
 
 struct MsState {
-    int iter, maxTerm, active, wpos;  // polled
-    double rNorm2, bnorm2;            // polled
-    int ns, max_iter, status, halt;
-    int nupd, wmax, pad0, pad1;
+    int iter, maxTerm, wpos, wmax;  // polled
+    // whether iterations still run: iteration n of a chunk reads active[n & 1] throughout and its shift step writes
+    // active[1 - (n & 1)], so that no kernel reads a flag that one of its own blocks may be writing (the batched
+    // solver, whose shift step runs after every tile of the system has passed, uses active[0] alone)
+    int active[2], status, halt;    // polled
+    double rNorm2, bnorm2;          // polled
+    int ns, max_iter, pad0, pad1;
     unsigned ticket[4];
     double tol;
-    double Bm1, pAp, lambda2;
+    double b0, a0;  // B_0 of this iteration (first dslash), a_0 of this iteration (second dslash)
+    double Bm1, lambda2;
     double pp;  // |p0|^2, kept by the recurrence |p'|^2 = |r'|^2 + a0^2 |p|^2; <p0, A p0> = sigma0 |p0|^2 + |D p0|^2
     double shift[kMaxShift];  // reference semantics: shift[0] absolute, shift[j] = sigma_j - sigma_0
-    double a[kMaxShift], B[kMaxShift], Z[kMaxShift], Zm1[kMaxShift];
+    double a[kMaxShift], B[kMaxShift], Z[kMaxShift], Zm1[kMaxShift];  // as of the last shift step
     double c[kMaxShift], e[kMaxShift];           // p_k, x_k coefficients of p_k at the window start
     double d[kMaxShift][kWin], f[kMaxShift][kWin];  // coefficients of the ring residuals
     int mode, next_mode;  // batched solver: operator precision of this / the next iteration (0 FP64, 1 FP32, 2 HALF)
@@ -25,8 +30,9 @@ struct MsState {
     int *running;             // batched solver: systems still iterating (decremented when this one stops)
 };
 
-struct MsPoll {
-    int iter, maxTerm, active, wpos;
+struct MsPoll {  // the first words of MsState
+    int iter, maxTerm, wpos, wmax;
+    int active[2], status, halt;
     double rNorm2, bnorm2;
 };
 
