@@ -63,6 +63,32 @@ __global__ void __launch_bounds__(256) dslash_full_kernel(Geom g, int pv, LinkSe
     st_spinor<SP>(dst + p * half, pv, i, acc);
 }
 
+// The three forms above with S threads per site (dslash_site_split): dst = D src on parity p, or on both parities
+// (half > 0: full-lattice fields, blockIdx.y = p), or sigma * pvec - D src when pvec is given.
+template <int LP, int SP, int S>
+__global__ void __launch_bounds__(S *split_sites(S)) dslash_split_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
+                                                                         const char *__restrict__ src,
+                                                                         const char *__restrict__ pvec,
+                                                                         char *__restrict__ dst, size_t half, int p,
+                                                                         double sigma, const int *__restrict__ gate)
+{
+    if (gate && *gate == 0) return;
+    using T = typename Acc2<LP, SP>::T;
+    constexpr int NS = split_sites(S);
+    __shared__ T part[(S - 1) * 6 * NS];
+    const int i = blockIdx.x * NS + threadIdx.x % NS;
+    const int par = half ? (int)blockIdx.y : p;
+    T acc[6];
+    if (!dslash_site_split<LP, SP, T, S>(g, pv, fat, lng, src + (1 - par) * half, par, i, i < g.vh, part, acc)) return;
+    if (pvec) {
+        T pv6[6];
+        ld_spinor<SP>(pvec + par * half, pv, i, pv6);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) acc[k] = (T)sigma * pv6[k] - acc[k];
+    }
+    st_spinor<SP>(dst + par * half, pv, i, acc);
+}
+
 // HALF kernel: 0 one site per thread, 4 .. 7 two sites per thread in packed FP32 with 4 .. 7 resident 128-thread
 // CTAs per SM (KUQCD_HALF_DSLASH = site | pair4 | pair5 | pair6 | pair7).  Default pair7: the kernel is latency-
 // bound, and 28 warps per SM at 72 registers (40 B of spills) beat 20 at 96 (48^3x96: 536 against 577 us).
@@ -89,12 +115,40 @@ static bool pair_ok(int lp, int sp)
     else if (LPv == P16 && SPv == P16) { constexpr int LP = 2, SP = 2; CALL; } \
     else { constexpr int LP = 2, SP = 1; CALL; }
 
+// Threads per site of a launch over `sites` output sites.  The HALF kernels spend as long on decoding as on loading
+// and gain from more threads as far as the FP32 ones (16^4: one thread per site 8.2 us, four 6.1 us).
+static int threads_per_site(int lp, int sites) { return split_of(sites, lp == P64 ? kSplitLimit64 : kSplitLimit32); }
+
+template <int LP, int SP>
+static cudaError_t launch_split(int S, const Geom &g, const GaugeDev &gd, const void *src, const void *pvec, void *dst,
+                                size_t half, int p, double sigma, const int *gate, cudaStream_t s)
+{
+    const int ns = split_sites(S);
+    const dim3 grid((g.vh + ns - 1) / ns, half ? 2 : 1);
+    const int pv = pad_sites(g.vh), bs = S * ns;
+    auto a = static_cast<const char *>(src);
+    auto b = static_cast<const char *>(pvec);
+    auto d = static_cast<char *>(dst);
+#define KQ_SPLIT(SV) \
+    dslash_split_kernel<LP, SP, SV><<<grid, bs, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], a, b, d, half, p, sigma, gate)
+    if (S == 2) KQ_SPLIT(2);
+    else if (S == 4) KQ_SPLIT(4);
+    else KQ_SPLIT(8);
+#undef KQ_SPLIT
+    return cudaGetLastError();
+}
+
 cudaError_t launch_dslash2(const Geom &g, const GaugeDev &gd, int lp, int sp, const void *src, void *dst,
                            int dst_parity, const int *gate, cudaStream_t s, int block)
 {
     if (!gd.have[lp] || !pair_ok(lp, sp)) {
         set_last_error("dslash: links not resident in the requested precision, or unsupported precision pair");
         return cudaErrorInvalidValue;
+    }
+    if (const int S = threads_per_site(lp, g.vh); S > 1 && block <= 0) {
+        cudaError_t e = cudaSuccess;
+        KQ_DISPATCH_PAIR(lp, sp, e = (launch_split<LP, SP>(S, g, gd, src, nullptr, dst, 0, dst_parity, 0.0, gate, s)));
+        return e;
     }
     const int pv = pad_sites(g.vh);
     if (lp == P16 && sp == P16 && !gate && half_kernel() != 0) {
@@ -133,6 +187,10 @@ cudaError_t launch_mdagm2(const Geom &g, const GaugeDev &gd, int lp, int sp, dou
 {
     cudaError_t e = launch_dslash2(g, gd, lp, sp, src, tmp, 1 - parity, nullptr, s, 0);
     if (e != cudaSuccess) return e;
+    if (const int S = threads_per_site(lp, g.vh); S > 1) {
+        KQ_DISPATCH_PAIR(lp, sp, e = (launch_split<LP, SP>(S, g, gd, tmp, src, dst, 0, parity, sigma, nullptr, s)));
+        return e;
+    }
     const int bs = 256;
     const int nb = (g.vh + bs - 1) / bs;
     const int pv = pad_sites(g.vh);
@@ -155,9 +213,14 @@ cudaError_t launch_dslash_full(const Geom &g, const GaugeDev &gd, int prec, cons
         set_last_error("dslash: links not resident in the requested precision");
         return cudaErrorInvalidValue;
     }
+    const size_t half = spinor_bytes(g, prec);
+    if (const int S = threads_per_site(prec, 2 * g.vh); S > 1) {
+        cudaError_t e = cudaSuccess;
+        KQ_DISPATCH_PAIR(prec, prec, e = (launch_split<LP, SP>(S, g, gd, src, pvec, dst, half, 0, sigma, nullptr, s)));
+        return e;
+    }
     const dim3 grid((g.vh + 255) / 256, 2);
     const int pv = pad_sites(g.vh);
-    const size_t half = spinor_bytes(g, prec);
     auto S = static_cast<const char *>(src);
     auto Pv = static_cast<const char *>(pvec);
     auto D = static_cast<char *>(dst);

@@ -217,6 +217,80 @@ __device__ __forceinline__ void dslash_site_t(const Geom &g, int pv, const LinkS
     fold_scale_site<LP>(fat, acc);
 }
 
+// Split form, for lattices whose sites alone do not fill the GPU: S threads share an output site, each taking 16 / S
+// terms of the sum (S = 2: two directions, 4: one direction, 8: one direction's forward or backward pair); thread
+// sub * NS + s of a CTA of S * NS threads works on site s of the CTA's NS, so a warp still reads 32 consecutive
+// sites of every plane.  The partial sums meet in shared memory and are added in the order of sub.  One thread per
+// site is a chain of sixteen link loads in too few warps to hide them: at 8^4 (8 CTAs) the FP64 dslash took 9.5 us for
+// 4 MB of links, with S = 8 3.3 us; at 16^4 14.0 us, with S = 2 9.3 us.
+// Sites per CTA for a given S.
+__host__ __device__ constexpr int split_sites(int S) { return S == 2 ? 64 : 32; }
+
+// Threads per site for vh sites: the most (up to 8) that keep vh * S within `limit` threads.  Beyond about 100,000
+// FP64 threads (of the 150,000 that fit at 64 registers) the extra CTAs only add partial sums: 16^3 x 32 took 21.3 us
+// with S = 1 and 23.4 us with S = 2 (FP32: 12.2 and 8.8 us, 24^4 25.4 and 31.2 us).
+constexpr int kSplitLimit64 = 100000, kSplitLimit32 = 150000;
+inline int split_of(int vh, int limit) { return vh <= limit / 8 ? 8 : vh <= limit / 4 ? 4 : vh <= limit / 2 ? 2 : 1; }
+
+// the two terms (fat hop 1, long hop 3) of direction dir and sign `sgn`; fat_b / lng_b: the parity whose links they use
+template <int LP, int SP, typename T>
+__device__ __forceinline__ void dslash_hop_pair(const Geom &g, int pv, const LinkSet &fat, const LinkSet &lng,
+                                                const void *fat_b, const void *lng_b, const void *src,
+                                                const SiteCoord &c, int i, int dir, int sgn, T rl, T acc[6])
+{
+    const int n1 = nbr_index(g, c, i, dir, sgn), n3 = nbr_index(g, c, i, dir, 3 * sgn);
+    T u[18], v[6];
+    ld_link_fold<LP>(fat_b, pv, dir, sgn > 0 ? i : n1, fat, u);
+    ld_spinor_as<SP>(src, pv, n1, v);
+    if (sgn > 0) mv_add(u, v, acc);
+    else mdv_sub(u, v, acc);
+    ld_link_fold<LP>(lng_b, pv, dir, sgn > 0 ? i : n3, lng, u);
+    ld_spinor_as<SP>(src, pv, n3, v);
+    fold_long_spinor<LP>(rl, v);
+    if (sgn > 0) mv_add(u, v, acc);
+    else mdv_sub(u, v, acc);
+}
+
+// acc = (D src)(i) in the threads of sub 0, which return true if `valid` (the site exists); every thread of the CTA
+// calls this.  part: (S - 1) * 6 * NS values of shared memory.
+template <int LP, int SP, typename T, int S>
+__device__ __forceinline__ bool dslash_site_split(const Geom &g, int pv, const LinkSet &fat, const LinkSet &lng,
+                                                  const void *src, int p, int i, bool valid, T *part, T acc[6])
+{
+    static_assert(S == 2 || S == 4 || S == 8, "threads per site");
+    constexpr int NS = split_sites(S);
+    const int sub = threadIdx.x / NS, s = threadIdx.x % NS;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) acc[k] = T(0);
+    if (valid) {
+        const SiteCoord c = site_coord(g, i, p);
+        const void *fat_p = p ? fat.par[1] : fat.par[0], *fat_q = p ? fat.par[0] : fat.par[1];
+        const void *lng_p = p ? lng.par[1] : lng.par[0], *lng_q = p ? lng.par[0] : lng.par[1];
+        const T rl = fold_scale_long<LP, T>(fat, lng);
+        constexpr int ND = S == 2 ? 2 : 1;  // directions per thread
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            const int dir = S == 8 ? sub >> 1 : ND * sub + d;
+            if (S < 8 || !(sub & 1))
+                dslash_hop_pair<LP, SP, T>(g, pv, fat, lng, fat_p, lng_p, src, c, i, dir, 1, rl, acc);
+            if (S < 8 || (sub & 1))
+                dslash_hop_pair<LP, SP, T>(g, pv, fat, lng, fat_q, lng_q, src, c, i, dir, -1, rl, acc);
+        }
+    }
+    if (sub) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) part[((sub - 1) * 6 + k) * NS + s] = acc[k];
+    }
+    __syncthreads();
+    if (sub) return false;
+#pragma unroll
+    for (int r = 0; r < S - 1; ++r)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) acc[k] += part[(r * 6 + k) * NS + s];
+    fold_scale_site<LP>(fat, acc);
+    return valid;
+}
+
 // Multi-RHS form: the links of site i are loaded once and applied to R right-hand sides whose fields are
 // src0 + sys[r] * stride (sys[r] < 0: slot unused).  acc[r] receives (D src_r)(i).
 template <int LP, int SP, int R>

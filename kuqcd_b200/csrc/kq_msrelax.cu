@@ -89,22 +89,41 @@ __global__ void __launch_bounds__(kBSm) ms_init_kernel(int vh, int pv, const voi
     }
 }
 
+// threads per CTA and sites per CTA of the dslash steps with S threads per site
+__host__ __device__ constexpr int ms_threads(int S) { return S == 1 ? kBSm : S * split_sites(S); }
+__host__ __device__ constexpr int ms_sites(int S) { return S == 1 ? kBSm : split_sites(S); }
+
+// acc = (D src)(i) for this thread's output site i of parity p; false in threads without one
+template <int LP, int SP, typename T, int S>
+__device__ __forceinline__ bool ms_site(const Geom &g, int pv, const LinkSet &fat, const LinkSet &lng, const void *src,
+                                        int p, int &i, T acc[6])
+{
+    i = blockIdx.x * ms_sites(S) + threadIdx.x % ms_sites(S);
+    if constexpr (S == 1) {
+        if (i >= g.vh) return false;
+        dslash_site_t<LP, SP, T>(g, pv, fat, lng, src, p, i, acc);
+        return true;
+    } else {
+        __shared__ T part[(S - 1) * 6 * ms_sites(S)];
+        return dslash_site_split<LP, SP, T, S>(g, pv, fat, lng, src, p, i, i < g.vh, part, acc);
+    }
+}
+
 // K1: tmp = D p0 (p0 FP64; links LP; tmp stored in SO); |tmp|^2, then the beta step with
 // <p0, A p0> = sigma0 |p0|^2 + |tmp|^2 (|p0|^2 from the alpha step's recurrence).  slot: parity of the iteration
-// within its chunk.
-template <int LP, int SO>
-__global__ void __launch_bounds__(kBSm) ms_dslash1_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
+// within its chunk.  S > 1: S threads per site (dslash_site_split).
+template <int LP, int SO, int S>
+__global__ void __launch_bounds__(ms_threads(S)) ms_dslash1_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
                                                           const void *__restrict__ p0, void *__restrict__ tmp, int q,
                                                           int slot, MsState *st, double *partials)
 {
     if (st->active[slot] == 0) return;
     __shared__ double sm[32];
-    const int i = blockIdx.x * kBSm + threadIdx.x;
+    typedef typename Acc2<LP, LP>::T T;
+    T acc[6];
     double tt = 0.0;
-    if (i < g.vh) {
-        typedef typename Acc2<LP, LP>::T T;
-        T acc[6];
-        dslash_site_t<LP, 0, T>(g, pv, fat, lng, p0, q, i, acc);
+    int i;
+    if (ms_site<LP, 0, T, S>(g, pv, fat, lng, p0, q, i, acc)) {
         st_spinor_as<SO>(tmp, pv, i, acc);
 #pragma unroll
         for (int k = 0; k < 6; ++k) tt += (double)acc[k] * (double)acc[k];
@@ -120,8 +139,8 @@ __global__ void __launch_bounds__(kBSm) ms_dslash1_kernel(Geom g, int pv, LinkSe
 
 // K2: s = sigma0 p0 - D tmp (tmp stored in SI, links LP; s stays in registers); r^(i+1) = r^(i) + B0 s into the
 // ring; |r|^2, then the alpha step
-template <int LP, int SI>
-__global__ void __launch_bounds__(kBSm) ms_dslash2_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
+template <int LP, int SI, int S>
+__global__ void __launch_bounds__(ms_threads(S)) ms_dslash2_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
                                                           const void *__restrict__ tmp, const void *__restrict__ p0,
                                                           char *ring, size_t vb, int p, int slot,
                                                           MsState *st, double *partials)
@@ -131,12 +150,11 @@ __global__ void __launch_bounds__(kBSm) ms_dslash2_kernel(Geom g, int pv, LinkSe
     const int it = st->iter;  // iterations completed before this one
     const char *rin = ring + (size_t)(it % kWin) * vb;
     char *rout = ring + (size_t)((it + 1) % kWin) * vb;
-    const int i = blockIdx.x * kBSm + threadIdx.x;
+    typedef typename Acc2<LP, LP>::T T;
+    T acc[6];
     double nn = 0.0;
-    if (i < g.vh) {
-        typedef typename Acc2<LP, LP>::T T;
-        T acc[6];
-        dslash_site_t<LP, SI, T>(g, pv, fat, lng, tmp, p, i, acc);
+    int i;
+    if (ms_site<LP, SI, T, S>(g, pv, fat, lng, tmp, p, i, acc)) {
         double pv6[6], rv[6];
         ld_spinor<0>(p0, pv, i, pv6);
         ld_spinor<0>(rin, pv, i, rv);
@@ -233,15 +251,35 @@ static int window_unroll()
 }
 
 // ---------------------------------------------------------------------------------------------------- driver
-template <int LP, int SO>
+// Threads per site of the dslash steps.  The FP64 and FP32 ones gain as the stand-alone kernels do (16^4: FP64 18.5
+// us with one thread per site and 14.4 with two, FP32 14.0 and, with four, 9.3 us); the HALF ones, short beside their
+// reduction, only on smaller lattices (12^4: 8.9 and, with four, 7.3 us; 16^4: 9.5 us with one thread, 9.6 with two).
+static int ms_split(int lp, int vh)
+{
+    return split_of(vh, lp == P64 ? kSplitLimit64 : lp == P32 ? kSplitLimit32 : 65000);
+}
+
+template <int LP, int S>
+static void enqueue_ms_dslash(const Geom &g, const GaugeDev &gd, const MsBuffers &w, int parity, int it, cudaStream_t s)
+{
+    const int pv = pad_sites(g.vh), nb = (g.vh + ms_sites(S) - 1) / ms_sites(S);
+    ms_dslash1_kernel<LP, LP, S><<<nb, ms_threads(S), 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.p0, w.tmp, 1 - parity,
+                                                              it & 1, w.st, w.partials);
+    ms_dslash2_kernel<LP, LP, S><<<nb, ms_threads(S), 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.tmp, w.p0,
+                                                              (char *)w.ring, w.vb, parity, it & 1, w.st, w.partials);
+}
+
+template <int LP>
 static void enqueue_ms_chunk(const Geom &g, const GaugeDev &gd, const MsBuffers &w, int parity, cudaStream_t s)
 {
     const int pv = pad_sites(g.vh), nb = (g.vh + kBSm - 1) / kBSm;
     for (int it = 0; it < kChunk; ++it) {
-        ms_dslash1_kernel<LP, SO><<<nb, kBSm, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.p0, w.tmp, 1 - parity, it & 1, w.st,
-                                                      w.partials);
-        ms_dslash2_kernel<LP, SO><<<nb, kBSm, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.tmp, w.p0, (char *)w.ring,
-                                                      w.vb, parity, it & 1, w.st, w.partials);
+        switch (ms_split(LP, g.vh)) {
+            case 8: enqueue_ms_dslash<LP, 8>(g, gd, w, parity, it, s); break;
+            case 4: enqueue_ms_dslash<LP, 4>(g, gd, w, parity, it, s); break;
+            case 2: enqueue_ms_dslash<LP, 2>(g, gd, w, parity, it, s); break;
+            default: enqueue_ms_dslash<LP, 1>(g, gd, w, parity, it, s); break;
+        }
         ms_p0_kernel<<<nb + 1, kBSm, 0, s>>>(g.vh, pv, (const char *)w.ring, w.vb, w.p0, it & 1, w.st);
     }
     switch (window_unroll()) {
@@ -262,7 +300,7 @@ size_t ms_workspace_bytes(const Geom &g, int ns)
 void ms_layout(Carve &c, const Geom &g, int ns, const void *d_b, void *d_x, MsBuffers &w)
 {
     const size_t vb = spinor_bytes(g, P64);
-    const int nb = (g.vh + kBSm - 1) / kBSm;
+    const int nb = (g.vh + 31) / 32;  // the most blocks a reduction kernel has (32 sites per CTA)
     w.vb = vb;
     w.b = d_b;
     w.x = d_x;
@@ -307,9 +345,9 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
         if ((m == 1 && !use32) || (m == 2 && !use16)) continue;
         cudaGraph_t graph = nullptr;
         KQ_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        if (m == 0) enqueue_ms_chunk<0, 0>(g, ctx->gd, w, parity, s);
-        else if (m == 1) enqueue_ms_chunk<1, 1>(g, ctx->gd, w, parity, s);
-        else enqueue_ms_chunk<2, 2>(g, ctx->gd, w, parity, s);
+        if (m == 0) enqueue_ms_chunk<0>(g, ctx->gd, w, parity, s);
+        else if (m == 1) enqueue_ms_chunk<1>(g, ctx->gd, w, parity, s);
+        else enqueue_ms_chunk<2>(g, ctx->gd, w, parity, s);
         cudaError_t ee = cudaStreamEndCapture(s, &graph);
         if (ee == cudaSuccess) ee = cudaGraphInstantiate(&exec[m], graph, 0);
         if (graph) cudaGraphDestroy(graph);
