@@ -222,7 +222,6 @@ __global__ void __launch_bounds__(BS) bk_init_kernel(const int2 *__restrict__ it
             st_spinor<0>(d.p0, d.pv, i, v);
             char *ring = static_cast<char *>(d.ring);
             st_spinor<0>(ring, d.pv, i, v);
-            for (int l = 1; l < kWin; ++l) st_spinor<0>(ring + l * d.vb, d.pv, i, z);
             for (int k = 0; k < st->ns; ++k) {
                 st_spinor<0>(static_cast<char *>(d.pw) + k * d.vb, d.pv, i, v);
                 st_spinor<0>(static_cast<char *>(d.x) + k * d.vb, d.pv, i, z);

@@ -55,8 +55,7 @@ __global__ void __launch_bounds__(kBSm) ms_init_kernel(int vh, int pv, const voi
         double v[6], z[6] = {0, 0, 0, 0, 0, 0};
         ld_spinor<0>(b, pv, i, v);
         st_spinor<0>(p0, pv, i, v);
-        st_spinor<0>(ring, pv, i, v);  // r^(0) in slot 0
-        for (int l = 1; l < kWin; ++l) st_spinor<0>(ring + l * vb, pv, i, z);
+        st_spinor<0>(ring, pv, i, v);  // r^(0) in slot 0; the other slots are written before they are read
         for (int k = 0; k < ns; ++k) {
             st_spinor<0>(pw0 + k * vb, pv, i, v);
             st_spinor<0>(x0 + k * vb, pv, i, z);
