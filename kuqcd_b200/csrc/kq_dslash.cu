@@ -10,8 +10,8 @@
 
 namespace kq {
 
-template <int LP, int SP>
-__global__ void __launch_bounds__(256) dslash_kernel(Geom g, int pv, LinkSet fat, LinkSet lng, const void *__restrict__ src,
+template <int LP, int SP, int MB>
+__global__ void __launch_bounds__(256, MB) dslash_kernel(Geom g, int pv, LinkSet fat, LinkSet lng, const void *__restrict__ src,
                                                      void *__restrict__ dst, int p, const int *__restrict__ gate)
 {
     if (gate && *gate == 0) return;
@@ -23,8 +23,8 @@ __global__ void __launch_bounds__(256) dslash_kernel(Geom g, int pv, LinkSet fat
 }
 
 // s = sigma * pvec - D src   (pvec, s on parity p)
-template <int LP, int SP>
-__global__ void __launch_bounds__(256) dslash_xmy_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
+template <int LP, int SP, int MB>
+__global__ void __launch_bounds__(256, MB) dslash_xmy_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
                                                          const void *__restrict__ src, const void *__restrict__ pvec,
                                                          void *__restrict__ s, int p, double sigma)
 {
@@ -43,8 +43,8 @@ __global__ void __launch_bounds__(256) dslash_xmy_kernel(Geom g, int pv, LinkSet
 // parity-1 field, `half` bytes apart.  blockIdx.y = output parity p; the input is the other half.  dst = D src on
 // both parities in one launch (dirac_hisq.cpp:128-136, 418-424 with offseti = offsetg = 0), or, with pvec,
 // dst = sigma * pvec - D src (the second half of sigma - D D).
-template <int LP, int SP>
-__global__ void __launch_bounds__(256) dslash_full_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
+template <int LP, int SP, int MB>
+__global__ void __launch_bounds__(256, MB) dslash_full_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
                                                           const char *__restrict__ src, const char *__restrict__ pvec,
                                                           char *__restrict__ dst, size_t half, double sigma)
 {
@@ -115,9 +115,18 @@ static bool pair_ok(int lp, int sp)
     else if (LPv == P16 && SPv == P16) { constexpr int LP = 2, SP = 2; CALL; } \
     else { constexpr int LP = 2, SP = 1; CALL; }
 
-// Threads per site of a launch over `sites` output sites.  The HALF kernels spend as long on decoding as on loading
-// and gain from more threads as far as the FP32 ones (16^4: one thread per site 8.2 us, four 6.1 us).
-static int threads_per_site(int lp, int sites) { return split_of(sites, lp == P64 ? kSplitLimit64 : kSplitLimit32); }
+static int threads_per_site(int lp, int sites)
+{
+    return split_of(sites, lp == P64 ? kSplitLimit64 : lp == P32 ? kSplitLimit32 : kSplitLimit16);
+}
+
+// CALL with MB = the resident CTAs per SM of a one-thread-per-site launch over `sites` output sites
+#define KQ_WITH_CTAS(LPv, sites, CALL)                              \
+    if (LPv == 0 && fp64_four_ctas(sites)) {                        \
+        constexpr int MB = LPv == 0 ? 4 : SiteCtas<LPv>::v; CALL;   \
+    } else {                                                        \
+        constexpr int MB = SiteCtas<LPv>::v; CALL;                  \
+    }
 
 template <int LP, int SP>
 static cudaError_t launch_split(int S, const Geom &g, const GaugeDev &gd, const void *src, const void *pvec, void *dst,
@@ -151,8 +160,9 @@ cudaError_t launch_dslash2(const Geom &g, const GaugeDev &gd, int lp, int sp, co
         return e;
     }
     const int pv = pad_sites(g.vh);
-    if (lp == P16 && sp == P16 && !gate && half_kernel() != 0) {
-        // HALF: two sites per thread in packed FP32 (kq_dslash_half2.cuh)
+    // HALF: two sites per thread in packed FP32 (kq_dslash_half2.cuh) on lattices of some waves of it; below, one site
+    // per thread is ahead (80,000 sites 12.6 against 13.2 us, 165,888 21.7 against 21.6 us)
+    if (lp == P16 && sp == P16 && !gate && half_kernel() != 0 && g.vh > 150000) {
         constexpr int kBS2 = 128;
         const int nb2 = (g.vh + 2 * kBS2 - 1) / (2 * kBS2);
         switch (half_kernel()) {
@@ -165,8 +175,8 @@ cudaError_t launch_dslash2(const Geom &g, const GaugeDev &gd, int lp, int sp, co
     }
     const int bs = block > 0 ? block : 256;
     const int nb = (g.vh + bs - 1) / bs;
-    KQ_DISPATCH_PAIR(lp, sp, (dslash_kernel<LP, SP><<<nb, bs, 0, s>>>(g, pv, gd.fat[lp], gd.lng[lp], src, dst,
-                                                                       dst_parity, gate)));
+    KQ_DISPATCH_PAIR(lp, sp, KQ_WITH_CTAS(LP, g.vh, (dslash_kernel<LP, SP, MB><<<nb, bs, 0, s>>>(
+                                 g, pv, gd.fat[lp], gd.lng[lp], src, dst, dst_parity, gate))));
     return cudaGetLastError();
 }
 
@@ -194,8 +204,8 @@ cudaError_t launch_mdagm2(const Geom &g, const GaugeDev &gd, int lp, int sp, dou
     const int bs = 256;
     const int nb = (g.vh + bs - 1) / bs;
     const int pv = pad_sites(g.vh);
-    KQ_DISPATCH_PAIR(lp, sp, (dslash_xmy_kernel<LP, SP><<<nb, bs, 0, s>>>(g, pv, gd.fat[lp], gd.lng[lp], tmp, src,
-                                                                           dst, parity, sigma)));
+    KQ_DISPATCH_PAIR(lp, sp, KQ_WITH_CTAS(LP, g.vh, (dslash_xmy_kernel<LP, SP, MB><<<nb, bs, 0, s>>>(
+                                 g, pv, gd.fat[lp], gd.lng[lp], tmp, src, dst, parity, sigma))));
     return cudaGetLastError();
 }
 
@@ -224,8 +234,8 @@ cudaError_t launch_dslash_full(const Geom &g, const GaugeDev &gd, int prec, cons
     auto S = static_cast<const char *>(src);
     auto Pv = static_cast<const char *>(pvec);
     auto D = static_cast<char *>(dst);
-    KQ_DISPATCH_PAIR(prec, prec, (dslash_full_kernel<LP, SP><<<grid, 256, 0, s>>>(g, pv, gd.fat[prec], gd.lng[prec],
-                                                                                  S, Pv, D, half, sigma)));
+    KQ_DISPATCH_PAIR(prec, prec, KQ_WITH_CTAS(LP, 2 * g.vh, (dslash_full_kernel<LP, SP, MB><<<grid, 256, 0, s>>>(
+                                     g, pv, gd.fat[prec], gd.lng[prec], S, Pv, D, half, sigma))));
     return cudaGetLastError();
 }
 

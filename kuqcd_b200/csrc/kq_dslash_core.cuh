@@ -226,11 +226,30 @@ __device__ __forceinline__ void dslash_site_t(const Geom &g, int pv, const LinkS
 // Sites per CTA for a given S.
 __host__ __device__ constexpr int split_sites(int S) { return S == 2 ? 64 : 32; }
 
-// Threads per site for vh sites: the most (up to 8) that keep vh * S within `limit` threads.  Beyond about 100,000
-// FP64 threads (of the 150,000 that fit at 64 registers) the extra CTAs only add partial sums: 16^3 x 32 took 21.3 us
-// with S = 1 and 23.4 us with S = 2 (FP32: 12.2 and 8.8 us, 24^4 25.4 and 31.2 us).
-constexpr int kSplitLimit64 = 100000, kSplitLimit32 = 150000;
-inline int split_of(int vh, int limit) { return vh <= limit / 8 ? 8 : vh <= limit / 4 ? 4 : vh <= limit / 2 ? 2 : 1; }
+// Threads per site for `sites` output sites: the most (up to 8) that keep sites * S within `limit` threads, about one
+// wave of the kernel (FP64 113,664 threads, FP32 189,440).  Beyond it the extra CTAs only add partial sums.  Measured
+// with S = 1 / 2 / 4 / 8 (us): FP64 12,096 sites 9.7 / 6.4 / 4.8 / 4.5, 24,192 10.8 / 7.7 / 8.7 / 7.9, 41,472 17.2 / 11.5
+// / 12.9 / 14.9, 52,488 20.0 / 22.3; FP32 24,192 8.4 / 5.8 / 4.7 / 5.0, 41,472 9.1 / 6.6 / 6.3 / 6.8, 80,000 15.0 / 11.0,
+// 120,000 20.6 / 22.8; HALF 19,208 6.3 / 5.4 / 4.7 / 5.1, 41,472 9.0 / 7.3 / 7.0 / 7.6, 65,536 9.2 / 9.4.
+constexpr int kSplitLimit64 = 94000, kSplitLimit32 = 175000, kSplitLimit16 = 150000;
+inline int split_of(int sites, int limit)
+{
+    return sites <= limit / 8 ? 8 : sites <= limit / 4 ? 4 : sites <= limit / 2 ? 2 : 1;
+}
+
+// Resident 256-thread CTAs per SM that the one-thread-per-site kernels are compiled for.  FP32: five (48 registers, as
+// without a bound; three or four at more registers are slower: 32^4 88 and 83 against 77 us).  HALF: four; without a
+// bound the compiler takes 44 registers, with too few loads in flight (solver kernels at 32^4: 72.6 and 84.7 us
+// unbounded, 64.3 and 70.0 us bounded).  FP64: three (80 registers; two to three per cent over no bound on lattices from
+// 16^4 to 48^4), but four where that saves the last of up to three waves: 120,000 sites are 1.06 waves of three CTAs
+// per SM and 0.79 of four, 47.4 and 38.5 us; 240,000 on a full lattice 77.9 and 69.0 us.
+template <int LP> struct SiteCtas { static constexpr int v = LP == 0 ? 3 : LP == 1 ? 5 : 4; };
+inline bool fp64_four_ctas(int sites)
+{
+    constexpr int wave3 = 148 * 3 * 256, wave4 = 148 * 4 * 256;
+    const int w3 = (sites + wave3 - 1) / wave3, w4 = (sites + wave4 - 1) / wave4;
+    return w3 <= 3 && w4 < w3;
+}
 
 // the two terms (fat hop 1, long hop 3) of direction dir and sign `sgn`; fat_b / lng_b: the parity whose links they use
 template <int LP, int SP, typename T>

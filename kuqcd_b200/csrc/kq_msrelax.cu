@@ -111,8 +111,8 @@ __device__ __forceinline__ bool ms_site(const Geom &g, int pv, const LinkSet &fa
 // K1: tmp = D p0 (p0 FP64; links LP; tmp stored in SO); |tmp|^2, then the beta step with
 // <p0, A p0> = sigma0 |p0|^2 + |tmp|^2 (|p0|^2 from the alpha step's recurrence).  slot: parity of the iteration
 // within its chunk.  S > 1: S threads per site (dslash_site_split).
-template <int LP, int SO, int S>
-__global__ void __launch_bounds__(ms_threads(S)) ms_dslash1_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
+template <int LP, int SO, int S, int MB>
+__global__ void __launch_bounds__(ms_threads(S), MB) ms_dslash1_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
                                                           const void *__restrict__ p0, void *__restrict__ tmp, int q,
                                                           int slot, MsState *st, double *partials)
 {
@@ -138,8 +138,8 @@ __global__ void __launch_bounds__(ms_threads(S)) ms_dslash1_kernel(Geom g, int p
 
 // K2: s = sigma0 p0 - D tmp (tmp stored in SI, links LP; s stays in registers); r^(i+1) = r^(i) + B0 s into the
 // ring; |r|^2, then the alpha step
-template <int LP, int SI, int S>
-__global__ void __launch_bounds__(ms_threads(S)) ms_dslash2_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
+template <int LP, int SI, int S, int MB>
+__global__ void __launch_bounds__(ms_threads(S), MB) ms_dslash2_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
                                                           const void *__restrict__ tmp, const void *__restrict__ p0,
                                                           char *ring, size_t vb, int p, int slot,
                                                           MsState *st, double *partials)
@@ -258,13 +258,15 @@ static int ms_split(int lp, int vh)
     return split_of(vh, lp == P64 ? kSplitLimit64 : lp == P32 ? kSplitLimit32 : 65000);
 }
 
-template <int LP, int S>
+// MB: resident CTAs per SM the kernels are compiled for (0: no bound, best for S > 1: at one the compiler takes 112
+// registers for FP64, S = 2 and the 16^4 solve goes from 12.8 to 13.9 ms)
+template <int LP, int S, int MB>
 static void enqueue_ms_dslash(const Geom &g, const GaugeDev &gd, const MsBuffers &w, int parity, int it, cudaStream_t s)
 {
     const int pv = pad_sites(g.vh), nb = (g.vh + ms_sites(S) - 1) / ms_sites(S);
-    ms_dslash1_kernel<LP, LP, S><<<nb, ms_threads(S), 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.p0, w.tmp, 1 - parity,
+    ms_dslash1_kernel<LP, LP, S, MB><<<nb, ms_threads(S), 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.p0, w.tmp, 1 - parity,
                                                               it & 1, w.st, w.partials);
-    ms_dslash2_kernel<LP, LP, S><<<nb, ms_threads(S), 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.tmp, w.p0,
+    ms_dslash2_kernel<LP, LP, S, MB><<<nb, ms_threads(S), 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.tmp, w.p0,
                                                               (char *)w.ring, w.vb, parity, it & 1, w.st, w.partials);
 }
 
@@ -274,10 +276,13 @@ static void enqueue_ms_chunk(const Geom &g, const GaugeDev &gd, const MsBuffers 
     const int pv = pad_sites(g.vh), nb = (g.vh + kBSm - 1) / kBSm;
     for (int it = 0; it < kChunk; ++it) {
         switch (ms_split(LP, g.vh)) {
-            case 8: enqueue_ms_dslash<LP, 8>(g, gd, w, parity, it, s); break;
-            case 4: enqueue_ms_dslash<LP, 4>(g, gd, w, parity, it, s); break;
-            case 2: enqueue_ms_dslash<LP, 2>(g, gd, w, parity, it, s); break;
-            default: enqueue_ms_dslash<LP, 1>(g, gd, w, parity, it, s); break;
+            case 8: enqueue_ms_dslash<LP, 8, 0>(g, gd, w, parity, it, s); break;
+            case 4: enqueue_ms_dslash<LP, 4, 0>(g, gd, w, parity, it, s); break;
+            case 2: enqueue_ms_dslash<LP, 2, 0>(g, gd, w, parity, it, s); break;
+            default:
+                if (LP == 0 && fp64_four_ctas(g.vh)) enqueue_ms_dslash<LP, 1, LP == 0 ? 4 : SiteCtas<LP>::v>(g, gd, w, parity, it, s);
+                else enqueue_ms_dslash<LP, 1, SiteCtas<LP>::v>(g, gd, w, parity, it, s);
+                break;
         }
         ms_p0_kernel<<<nb + 1, kBSm, 0, s>>>(g.vh, pv, (const char *)w.ring, w.vb, w.p0, it & 1, w.st);
     }
