@@ -23,12 +23,10 @@ const char *last_error() { return g_last_error.c_str(); }
 
 cudaError_t launch_mdagm(const Geom &g, const GaugeDev &gd, int prec, double sigma, const void *src, void *tmp,
                          void *dst, int parity, cudaStream_t s);
-cudaError_t true_residuals(const Geom &g, const GaugeDev &gd, int parity, int ns, const double *sigma,
-                           const void *d_b, const void *d_x, size_t xstride, void *d_tmp, void *d_s, double *partials,
-                           double *out, cudaStream_t s);
-cudaError_t true_residuals_full(const Geom &g, const GaugeDev &gd, int ns, const double *sigma, const void *d_b,
-                                const void *d_x, size_t xstride, void *d_tmp, void *d_s, double *partials,
-                                double *out, cudaStream_t s);
+size_t resid_partials_bytes(const Geom &g, int ns);
+cudaError_t residual_norms(const Geom &g, const GaugeDev &gd, int parity, int ns, const double *sigma, const void *d_b,
+                           const void *d_x, size_t xstride, void *tmp, int fields, double *partials, double *d_sums,
+                           double *sums, cudaStream_t s);
 cudaError_t launch_dslash_full(const Geom &g, const GaugeDev &gd, int prec, const void *src, const void *pvec,
                                void *dst, double sigma, cudaStream_t s);
 cudaError_t launch_mdagm_full(const Geom &g, const GaugeDev &gd, int prec, double sigma, const void *src, void *tmp,
@@ -443,22 +441,40 @@ KQ_API KuQCDStatus kq_true_residuals(kq_context *ctx, int parity, int num_shift,
         if (st != KUQCD_SUCCESS) return st;
     }
     cudaSetDevice(ctx->device);
-    const size_t vb = spinor_bytes(ctx->g, P64) * (full ? 2 : 1);
-    const int nb = (ctx->g.vh + 255) / 256;
-    Carve c(nullptr);
-    c.take(vb);
-    c.take(vb);
-    c.take(sizeof(double) * 4 * nb);
-    cudaError_t e = ensure_work(ctx, c.off);
+    const size_t vb = spinor_bytes(ctx->g, P64);
+    const size_t pb = resid_partials_bytes(ctx->g, num_shift), sb = sizeof(double) * (kMaxShift + 1);
+    // temporaries for eight shifts at a time, or for the four that share a link load
+    int fields = std::min(num_shift, 8);
+    auto bytes = [&] {
+        Carve c(nullptr);
+        c.take(vb * fields);
+        c.take(pb);
+        c.take(sb);
+        return c.off;
+    };
+    cudaError_t e = ensure_work(ctx, bytes());
+    if (e == cudaErrorMemoryAllocation && fields > 4) {
+        cudaGetLastError();
+        fields = 4;
+        e = ensure_work(ctx, bytes());
+    }
     if (e != cudaSuccess) return status_of(e);
     Carve w(ctx->work);
-    void *tmp = w.take(vb), *s = w.take(vb);
-    double *partials = static_cast<double *>(w.take(sizeof(double) * 4 * nb));
-    if (full)
-        e = true_residuals_full(ctx->g, ctx->gd, num_shift, sigma, d_b, d_x, vb, tmp, s, partials, out, ctx->stream);
-    else
-        e = true_residuals(ctx->g, ctx->gd, parity, num_shift, sigma, d_b, d_x, vb, tmp, s, partials, out,
-                           ctx->stream);
+    void *tmp = w.take(vb * fields);
+    double *partials = static_cast<double *>(w.take(pb)), *d_sums = static_cast<double *>(w.take(sb));
+    double *sums = reinterpret_cast<double *>(ctx->poll);  // pinned
+    double rr[kMaxShift] = {0.0}, bb = 0.0;
+    // sigma - D D couples no parities: the full-lattice norms are the sums of the two halves'
+    for (int h = 0; h < (full ? 2 : 1) && e == cudaSuccess; ++h) {
+        e = residual_norms(ctx->g, ctx->gd, full ? h : parity, num_shift, sigma, static_cast<const char *>(d_b) + h * vb,
+                           static_cast<const char *>(d_x) + h * vb, full ? 2 * vb : vb, tmp, fields, partials, d_sums,
+                           sums, ctx->stream);
+        if (e != cudaSuccess) break;
+        for (int k = 0; k < num_shift; ++k) rr[k] += sums[k];
+        bb += sums[num_shift];
+    }
+    if (e == cudaSuccess)
+        for (int k = 0; k < num_shift; ++k) out[k] = bb > 0 ? std::sqrt(rr[k] / bb) : 0.0;
     return status_of(e);
 }
 

@@ -45,11 +45,15 @@ struct MrBuffers {
     void *r, *p, *xs, *ap, *tmp;  // FP32 sloppy vectors, vb32 apart
     void *tmp64;        // FP64, vb64 apart (other parity)
     size_t vb32, vb64;
-    double *partials;   // ns * site_blocks
+    double *partials;   // ns per site block of the kernel that writes them
     MrState *st;
 };
 
 constexpr int kBS = 256;
+// The FP64 kernels (residuals of the check and of every reliable update): four systems per thread in 128-thread CTAs,
+// three per SM, so that each link load serves four systems (12 systems at 32^4: 1.35 ms with two per thread in
+// 256-thread CTAs, 0.71 ms).
+constexpr int kBS64 = 128, kR64 = 4, kCtas64 = 3;
 
 template <int R>
 __device__ __forceinline__ void group_systems(const int *list, int n, int grp, int sys[R])
@@ -74,13 +78,6 @@ __device__ __forceinline__ bool last_block(unsigned *ticket)
     __syncthreads();
     if (last) __threadfence();
     return last;
-}
-
-__device__ __forceinline__ double sum_partials(const double *p, int n, double *sm)
-{
-    double s = 0.0;
-    for (int b = threadIdx.x; b < n; b += blockDim.x) s += ((volatile const double *)p)[b];
-    return block_sum(s, sm);
 }
 
 // ---------------------------------------------------------------------------------------------------- kernels
@@ -140,7 +137,7 @@ __global__ void __launch_bounds__(kBS) mr_dslash2_kernel(Geom g, int pv, LinkSet
     if (!last_block(&st->ticket[0])) return;
     for (int a = 0; a < n; ++a) {
         const int k = st->act[a];
-        const double pAp = sum_partials(partials + k * gridDim.y, gridDim.y, sm);
+        const double pAp = partials_sum(partials + (size_t)k * gridDim.y, gridDim.y, sm);
         if (threadIdx.x == 0) st->alpha[k] = st->rr[k] / pAp;
     }
     if (threadIdx.x == 0) st->ticket[0] = 0;
@@ -191,7 +188,7 @@ __global__ void __launch_bounds__(kBS) mr_update_kernel(int vh, int pv, const ch
     __syncthreads();
     for (int a = 0; a < n; ++a) {
         const int k = st->act[a];
-        const double rr = sum_partials(partials + k * gridDim.y, gridDim.y, sm);
+        const double rr = partials_sum(partials + (size_t)k * gridDim.y, gridDim.y, sm);
         if (threadIdx.x == 0) {
             st->sys_iter[k] += 1;
             if (rr < st->target2 || rr < st->delta2 * st->maxrr[k] || !isfinite(rr)) {
@@ -238,16 +235,17 @@ __global__ void __launch_bounds__(kBS) mr_accum_kernel(int vh, int pv, char *xs0
 
 // K5: tmp64_k = D x64_k (FP64, flagged systems, output parity q)
 template <int R>
-__global__ void __launch_bounds__(kBS) mr_dslash64_kernel(Geom g, int pv, LinkSet fat, LinkSet lng, const char *x640,
+__global__ void __launch_bounds__(kBS64, kCtas64) mr_dslash64_kernel(Geom g, int pv, LinkSet fat, LinkSet lng, const char *x640,
                                                           char *t640, size_t vb64, int q, const MrState *st)
 {
     int sys[R];
     group_systems<R>(st->flag, st->nflag, blockIdx.x, sys);
     if (sys[0] < 0) return;
-    const int i = blockIdx.y * kBS + threadIdx.x;
+    const int i = blockIdx.y * kBS64 + threadIdx.x;
     if (i >= g.vh) return;
     double acc[R][6];
-    dslash_site_mrhs<0, 0, R>(g, pv, fat, lng, x640, vb64, sys, q, i, acc);
+    if (sys[R - 1] >= 0) dslash_site_mrhs<0, 0, R, true>(g, pv, fat, lng, x640, vb64, sys, q, i, acc);
+    else dslash_site_mrhs<0, 0, R>(g, pv, fat, lng, x640, vb64, sys, q, i, acc);
 #pragma unroll
     for (int r = 0; r < R; ++r)
         if (sys[r] >= 0) st_spinor<0>(t640 + sys[r] * vb64, pv, i, acc[r]);
@@ -255,7 +253,7 @@ __global__ void __launch_bounds__(kBS) mr_dslash64_kernel(Geom g, int pv, LinkSe
 
 // K6: r_k = b - (sigma_k x64_k - D tmp64_k) in FP64, stored FP32 ; |r_k|^2 -> convergence or beta_k (flagged)
 template <int R>
-__global__ void __launch_bounds__(kBS) mr_resid_kernel(Geom g, int pv, LinkSet fat, LinkSet lng, const char *t640,
+__global__ void __launch_bounds__(kBS64, kCtas64) mr_resid_kernel(Geom g, int pv, LinkSet fat, LinkSet lng, const char *t640,
                                                        const char *x640, size_t vb64, const void *b, char *r0,
                                                        size_t vb, int parity, MrState *st, double *partials)
 {
@@ -264,13 +262,14 @@ __global__ void __launch_bounds__(kBS) mr_resid_kernel(Geom g, int pv, LinkSet f
     if (n == 0) return;
     int sys[R];
     group_systems<R>(st->flag, n, blockIdx.x, sys);
-    const int i = blockIdx.y * kBS + threadIdx.x;
+    const int i = blockIdx.y * kBS64 + threadIdx.x;
     double nn[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) nn[r] = 0.0;
     if (sys[0] >= 0 && i < g.vh) {
         double acc[R][6], bv[6];
-        dslash_site_mrhs<0, 0, R>(g, pv, fat, lng, t640, vb64, sys, parity, i, acc);
+        if (sys[R - 1] >= 0) dslash_site_mrhs<0, 0, R, true>(g, pv, fat, lng, t640, vb64, sys, parity, i, acc);
+        else dslash_site_mrhs<0, 0, R>(g, pv, fat, lng, t640, vb64, sys, parity, i, acc);
         ld_spinor<0>(b, pv, i, bv);
 #pragma unroll
         for (int r = 0; r < R; ++r)
@@ -297,7 +296,7 @@ __global__ void __launch_bounds__(kBS) mr_resid_kernel(Geom g, int pv, LinkSet f
     if (!last_block(&st->ticket[2])) return;
     for (int a = 0; a < n; ++a) {
         const int k = st->flag[a];
-        const double rr = sum_partials(partials + k * gridDim.y, gridDim.y, sm);
+        const double rr = partials_sum(partials + (size_t)k * gridDim.y, gridDim.y, sm);
         if (threadIdx.x == 0) {
             const double rel = sqrt(rr / st->bnorm2);
             st->res[k] = rel;
@@ -375,17 +374,16 @@ __global__ void __launch_bounds__(kBS) norm2_partials_kernel(int vh, int pv, con
 
 // ---------------------------------------------------------------------------------------------------- driver
 constexpr int kR = 4;    // systems per thread in the sloppy multi-RHS kernels
-constexpr int kR64 = 2;  // systems per thread in the FP64 reliable-update kernels
 
 template <int LP>
 static void enqueue_reliable(const Geom &g, const GaugeDev &gd, const MrBuffers &w, int parity, int ns, cudaStream_t s)
 {
     const int pv = pad_sites(g.vh), sb = (g.vh + kBS - 1) / kBS;
-    const dim3 g64((ns + kR64 - 1) / kR64, sb), gs((ns + kR - 1) / kR, sb);
+    const dim3 g64((ns + kR64 - 1) / kR64, (g.vh + kBS64 - 1) / kBS64), gs((ns + kR - 1) / kR, sb);
     mr_accum_kernel<kR><<<gs, kBS, 0, s>>>(g.vh, pv, (char *)w.xs, w.vb32, (char *)w.x64, w.vb64, w.st);
-    mr_dslash64_kernel<kR64><<<g64, kBS, 0, s>>>(g, pv, gd.fat[0], gd.lng[0], (const char *)w.x64, (char *)w.tmp64,
+    mr_dslash64_kernel<kR64><<<g64, kBS64, 0, s>>>(g, pv, gd.fat[0], gd.lng[0], (const char *)w.x64, (char *)w.tmp64,
                                                  w.vb64, 1 - parity, w.st);
-    mr_resid_kernel<kR64><<<g64, kBS, 0, s>>>(g, pv, gd.fat[0], gd.lng[0], (const char *)w.tmp64,
+    mr_resid_kernel<kR64><<<g64, kBS64, 0, s>>>(g, pv, gd.fat[0], gd.lng[0], (const char *)w.tmp64,
                                               (const char *)w.x64, w.vb64, w.b, (char *)w.r, w.vb32, parity, w.st,
                                               w.partials);
     mr_p_kernel<kR><<<gs, kBS, 0, s>>>(g.vh, pv, (const char *)w.r, (char *)w.p, w.vb32, w.st);
@@ -449,7 +447,7 @@ cudaError_t mixed_solve(::kq_context *ctx, const kq_solve_param *param, const do
     // ---- workspace
     auto layout = [&](Carve &c, MsBuffers &cw, MrBuffers &mw) {
         ms_layout(c, g, ns, d_b, d_x, cw);
-        mw.partials = static_cast<double *>(c.take(sizeof(double) * (size_t)sb * ns));
+        mw.partials = static_cast<double *>(c.take(sizeof(double) * (size_t)((g.vh + kBS64 - 1) / kBS64) * ns));
         mw.b = d_b;
         mw.x64 = d_x;
         mw.vb32 = vb32;
