@@ -470,6 +470,7 @@ cudaError_t mixed_solve(::kq_context *ctx, const kq_solve_param *param, const do
     layout(c, cw, mw);
     long long launches = 0;
 
+    MsResult r1;
     // ---- |b|^2
     {
         const int pv = pad_sites(g.vh);
@@ -525,7 +526,6 @@ cudaError_t mixed_solve(::kq_context *ctx, const kq_solve_param *param, const do
         const double rho16 = lp == P16 ? relax_frac * target / eps16 : 0.0;
         if (run_phase1) {
             NvtxRange nvtx("mixed: relaxed-precision multishift");
-            MsResult r1;
             KQ_CUDA_TRY(ms_solve(ctx, cw, param->parity, ns, rs, stop_frac * stop_frac * target * target * bb,
                                  param->max_iter > 0 ? param->max_iter : 100000, rho32, rho16, &r1));
             info->iter = r1.iter;
@@ -543,38 +543,49 @@ cudaError_t mixed_solve(::kq_context *ctx, const kq_solve_param *param, const do
     KQ_CUDA_TRY(cudaGetLastError());
     launches += 4;
 
+    // chunks of refinement iterations, the first enqueued kernel by kernel (most solves need no second), the others as
+    // a graph
     const int chunk = 4;
-    cudaGraph_t graph = nullptr;
+    auto enqueue_chunk = [&] {
+        for (int it = 0; it < chunk; ++it) {
+            if (lp == P32) enqueue_mr_iteration<1>(g, ctx->gd, mw, param->parity, ns, s);
+            else enqueue_mr_iteration<2>(g, ctx->gd, mw, param->parity, ns, s);
+        }
+    };
     cudaGraphExec_t exec = nullptr;
-    KQ_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    for (int it = 0; it < chunk; ++it) {
-        if (lp == P32) enqueue_mr_iteration<1>(g, ctx->gd, mw, param->parity, ns, s);
-        else enqueue_mr_iteration<2>(g, ctx->gd, mw, param->parity, ns, s);
-    }
-    cudaError_t ee = cudaStreamEndCapture(s, &graph);
-    if (ee != cudaSuccess) {
+    auto build = [&]() -> cudaError_t {
+        cudaGraph_t graph = nullptr;
+        KQ_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        enqueue_chunk();
+        cudaError_t ee = cudaStreamEndCapture(s, &graph);
+        if (ee == cudaSuccess) ee = cudaGraphInstantiate(&exec, graph, 0);
         if (graph) cudaGraphDestroy(graph);
-        set_last_error(std::string("mixed solver: graph capture failed: ") + cudaGetErrorString(ee));
+        if (ee != cudaSuccess)
+            set_last_error(std::string("mixed solver: graph build failed: ") + cudaGetErrorString(ee));
         return ee;
-    }
-    ee = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
-    KQ_CUDA_TRY(ee);
+    };
     // the pinned poll page receives the first four ints of MrState: nact, nflag, iter, max_iter
     int *poll = reinterpret_cast<int *>(ctx->poll);
     cudaError_t err = cudaSuccess;
     int replays = 0;
     const int hs_max_iter = param->max_iter > 0 ? param->max_iter : 100000;
     for (;;) {
-        KQ_CUDA_TRY(cudaMemcpyAsync(poll, mw.st, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
-        err = cudaStreamSynchronize(s);
+        err = cudaMemcpyAsync(poll, mw.st, 4 * sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(s);
         if (err != cudaSuccess || poll[0] == 0) break;  // no active system left
-        err = cudaGraphLaunch(exec, s);
+        if (replays == 0) {
+            enqueue_chunk();
+            err = cudaGetLastError();
+            r1.release();  // while the chunk runs
+        } else {
+            if (!exec) err = build();
+            if (err == cudaSuccess) err = cudaGraphLaunch(exec, s);
+        }
         if (err != cudaSuccess) break;
         launches += 7LL * chunk;
         if (++replays > hs_max_iter / chunk + 8) break;  // the refinement stops by then while its state is consistent
     }
-    cudaGraphExecDestroy(exec);
+    if (exec) cudaGraphExecDestroy(exec);
     KQ_CUDA_TRY(err);
     MrState hs;
     KQ_CUDA_TRY(cudaMemcpyAsync(&hs, mw.st, sizeof(hs), cudaMemcpyDeviceToHost, s));

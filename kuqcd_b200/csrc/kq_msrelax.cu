@@ -238,6 +238,21 @@ __global__ void __launch_bounds__(kBSm, 2) ms_window_kernel(int vh, int pv, cons
     }
 }
 
+// Writes the polled words of the state to the host page, chunk n to slot n & 1 (slots kPollSlot bytes apart).  A kernel
+// at the end of the chunk's graph: a copy behind it costs the GPU about 6 us more per chunk.
+constexpr int kPollSlot = 256;
+static_assert(sizeof(MsPoll) <= kPollSlot, "poll slot");
+__global__ void ms_poll_kernel(char *host, MsState *st)
+{
+    static_assert(sizeof(MsPoll) % sizeof(int) == 0, "copied by words");
+    const int slot = st->polls & 1;
+    __syncwarp();
+    volatile int *dst = reinterpret_cast<volatile int *>(host + slot * kPollSlot);
+    const int *src = reinterpret_cast<const int *>(st);
+    for (int t = threadIdx.x; t < (int)(sizeof(MsPoll) / sizeof(int)); t += 32) dst[t] = src[t];
+    if (threadIdx.x == 0) st->polls += 1;
+}
+
 // shifts updated per step of the window kernel's loop (KUQCD_WINDOW_UNROLL = 1 | 2 | 4)
 static int window_unroll()
 {
@@ -271,7 +286,8 @@ static void enqueue_ms_dslash(const Geom &g, const GaugeDev &gd, const MsBuffers
 }
 
 template <int LP>
-static void enqueue_ms_chunk(const Geom &g, const GaugeDev &gd, const MsBuffers &w, int parity, cudaStream_t s)
+static void enqueue_ms_chunk(const Geom &g, const GaugeDev &gd, const MsBuffers &w, int parity, char *host_poll,
+                             cudaStream_t s)
 {
     const int pv = pad_sites(g.vh), nb = (g.vh + kBSm - 1) / kBSm;
     for (int it = 0; it < kChunk; ++it) {
@@ -291,6 +307,15 @@ static void enqueue_ms_chunk(const Geom &g, const GaugeDev &gd, const MsBuffers 
         case 2: ms_window_kernel<2><<<nb, kBSm, 0, s>>>(g.vh, pv, (const char *)w.ring, w.vb, (char *)w.pw, (char *)w.x, w.st); break;
         default: ms_window_kernel<4><<<nb, kBSm, 0, s>>>(g.vh, pv, (const char *)w.ring, w.vb, (char *)w.pw, (char *)w.x, w.st); break;
     }
+    ms_poll_kernel<<<1, 32, 0, s>>>(host_poll, w.st);
+}
+
+static void enqueue_ms_chunk(int m, const Geom &g, const GaugeDev &gd, const MsBuffers &w, int parity, char *host_poll,
+                             cudaStream_t s)
+{
+    if (m == 0) enqueue_ms_chunk<0>(g, gd, w, parity, host_poll, s);
+    else if (m == 1) enqueue_ms_chunk<1>(g, gd, w, parity, host_poll, s);
+    else enqueue_ms_chunk<2>(g, gd, w, parity, host_poll, s);
 }
 
 size_t ms_workspace_bytes(const Geom &g, int ns)
@@ -343,28 +368,49 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
     KQ_CUDA_TRY(cudaGetLastError());
     long long launches = 1;
 
-    // one graph per operator precision, each W iterations + the window update
-    cudaGraphExec_t exec[3] = {nullptr, nullptr, nullptr};
-    for (int m = 0; m < 3; ++m) {
-        if ((m == 1 && !use32) || (m == 2 && !use16)) continue;
+    // One graph per operator precision, each kChunk iterations + the window update.  Building one takes the host about
+    // 130 us (and its first launch more): the first two chunks are enqueued kernel by kernel and the graphs built while
+    // they run.
+    cudaGraphExec_t *exec = res->exec;
+    char *host_poll = reinterpret_cast<char *>(ctx->poll);
+    auto build = [&](int m) -> cudaError_t {
         cudaGraph_t graph = nullptr;
         KQ_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        if (m == 0) enqueue_ms_chunk<0>(g, ctx->gd, w, parity, s);
-        else if (m == 1) enqueue_ms_chunk<1>(g, ctx->gd, w, parity, s);
-        else enqueue_ms_chunk<2>(g, ctx->gd, w, parity, s);
+        enqueue_ms_chunk(m, g, ctx->gd, w, parity, host_poll, s);
         cudaError_t ee = cudaStreamEndCapture(s, &graph);
         if (ee == cudaSuccess) ee = cudaGraphInstantiate(&exec[m], graph, 0);
         if (graph) cudaGraphDestroy(graph);
-        if (ee != cudaSuccess) {
-            for (auto &x : exec)
-                if (x) cudaGraphExecDestroy(x);
-            set_last_error(std::string("multishift: graph build failed: ") + cudaGetErrorString(ee));
-            return ee;
-        }
-    }
-    MsPoll *poll = reinterpret_cast<MsPoll *>(ctx->poll);
+        if (ee == cudaSuccess) ee = cudaGraphUpload(exec[m], s);
+        if (ee != cudaSuccess) set_last_error(std::string("multishift: graph build failed: ") + cudaGetErrorString(ee));
+        return ee;
+    };
+    // Up to two chunks are in flight: the one whose state the host waits for and, launched ahead of it, the next, so
+    // that the GPU does not idle through a poll and a graph launch after every kChunk iterations (35 us of a chunk's
+    // 170 us at 8^4).  The next chunk is launched ahead only where the last two states predict that the one in flight
+    // neither ends the solve nor reaches a switch of precision; a wrong guess costs a chunk of no-ops, or keeps the
+    // higher precision for kChunk more iterations.  The guess depends on the iterates alone, so a solve repeats
+    // exactly.
+    cudaEvent_t done[2] = {nullptr, nullptr};
     cudaError_t err = cudaSuccess;
+    for (auto &ev : done)
+        if (err == cudaSuccess) err = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     int chunks[3] = {0, 0, 0};
+    int launched = 0, polled = 0;
+    auto mode_of = [&](double rel2) { return use16 && rel2 < rho16 * rho16 ? 2 : use32 && rel2 < rho32 * rho32 ? 1 : 0; };
+    auto launch = [&](int m) {
+        if (err == cudaSuccess && launched >= 2 && !exec[m]) err = build(m);
+        if (err == cudaSuccess) {
+            if (exec[m]) err = cudaGraphLaunch(exec[m], s);
+            else {
+                enqueue_ms_chunk(m, g, ctx->gd, w, parity, host_poll, s);
+                err = cudaGetLastError();
+            }
+        }
+        if (err == cudaSuccess) err = cudaEventRecord(done[launched & 1], s);
+        chunks[m] += 1;
+        launched += 1;
+        launches += 3 * kChunk + 2;
+    };
     // Shifts k >= final_from have been reported final.  A shift dropped from the iteration (k >= maxTerm) receives
     // its last update in the next window flush; once the window is flushed (wpos = 0), x_k no longer changes.
     int final_from = ns;
@@ -373,31 +419,46 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
             for (int k = final_from - 1; k >= mt; --k) ctx->solution_ready(ctx, k, ctx->solution_ready_user);
         final_from = std::min(final_from, mt);
     };
-    for (;;) {
-        err = cudaMemcpyAsync(poll, w.st, sizeof(MsPoll), cudaMemcpyDeviceToHost, s);
-        if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+    const int most = max_iter / kChunk + 3;  // chunks: every solve has stopped by then while its state is consistent
+    double rel2 = 1.0, fall = 1e-2;  // |r|^2 / |b|^2 of the last state read, and its factor over the chunk before it
+    double stop2 = 0.0;              // the tolerance in the same units, once |b|^2 is known
+    launch(mode_of(rel2));
+    while (err == cudaSuccess) {
+        const int m = mode_of(rel2);
+        const double guess = rel2 * std::min(fall, 1.0);  // state after the chunk in flight
+        if (launched < most && guess > stop2 && mode_of(0.1 * guess) == m) launch(m);
+        // a graph that will be wanted, one per chunk in flight
+        for (int b : {m, use32 ? 1 : 0, use16 ? 2 : 0})
+            if (err == cudaSuccess && !exec[b] && b >= m) {
+                err = build(b);
+                break;
+            }
         if (err != cudaSuccess) break;
-        if (!poll->active[0]) {
-            if (poll->wpos == 0) report(0);  // stopped, last window flushed: every x_k is final
+        err = cudaEventSynchronize(done[polled & 1]);
+        if (err != cudaSuccess) break;
+        const MsPoll st = *reinterpret_cast<const MsPoll *>(host_poll + (polled & 1) * kPollSlot);
+        polled += 1;
+        if (!st.active[0]) {
+            if (st.wpos == 0) report(0);  // stopped, last window flushed: every x_k is final
             break;
         }
-        const int mt = poll->maxTerm, flushed = poll->wpos == 0;
-        const double rel2 = poll->rNorm2 / poll->bnorm2;
-        int m = 0;
-        if (use16 && rel2 < rho16 * rho16) m = 2;
-        else if (use32 && rel2 < rho32 * rho32) m = 1;
-        err = cudaGraphLaunch(exec[m], s);
-        if (err != cudaSuccess) break;
-        if (flushed) report(mt);  // the work it enqueues runs behind this chunk
-        chunks[m] += 1;
-        launches += 3 * kChunk + 1;
-        if (chunks[0] + chunks[1] + chunks[2] > max_iter / kChunk + 2) break;
+        const double now = st.rNorm2 / st.bnorm2;
+        fall = now / rel2;
+        rel2 = now;
+        stop2 = tol / st.bnorm2;
+        if (polled >= most) break;
+        if (launched == polled) launch(mode_of(rel2));
+        if (st.wpos == 0) report(st.maxTerm);  // the work it enqueues runs behind the chunks in flight
     }
-    for (auto &x : exec)
-        if (x) cudaGraphExecDestroy(x);
-    KQ_CUDA_TRY(err);
-    KQ_CUDA_TRY(cudaMemcpyAsync(&h, w.st, sizeof(MsState), cudaMemcpyDeviceToHost, s));
-    KQ_CUDA_TRY(cudaStreamSynchronize(s));
+    if (err == cudaSuccess) err = cudaMemcpyAsync(&h, w.st, sizeof(MsState), cudaMemcpyDeviceToHost, s);
+    const cudaError_t es = cudaStreamSynchronize(s);
+    for (auto &ev : done)
+        if (ev) cudaEventDestroy(ev);
+    if (err == cudaSuccess) err = es;
+    if (err != cudaSuccess) {
+        res->release();
+        KQ_CUDA_TRY(err);
+    }
     res->iter = h.iter;
     res->status = h.status ? h.status : (h.iter >= max_iter && h.maxTerm > 0 ? KQ_STATUS_MAXITER : 0);
     res->launches = launches;

@@ -15,7 +15,7 @@ struct MsState {
     // solver, whose shift step runs after every tile of the system has passed, uses active[0] alone)
     int active[2], status, halt;    // polled
     double rNorm2, bnorm2;          // polled
-    int ns, max_iter, pad0, pad1;
+    int ns, max_iter, polls, pad0;  // polls: chunks whose state has been written to the host
     unsigned ticket[4];
     double tol;
     double b0, a0;  // B_0 of this iteration (first dslash), a_0 of this iteration (second dslash)
@@ -46,9 +46,23 @@ struct MsBuffers {
 };
 
 struct MsResult {
-    int iter, status;
-    long long launches;
-    int chunks[3];  // chunks of kChunk iterations run with FP64 / FP32 / HALF operators
+    int iter = 0, status = 0;
+    long long launches = 0;
+    int chunks[3] = {0, 0, 0};  // chunks of kChunk iterations run with FP64 / FP32 / HALF operators
+    // the solve's graphs, destroyed with the result: destroying one takes the host 70 to 100 us, which a caller with
+    // more work for the GPU spends after enqueuing it
+    cudaGraphExec_t exec[3] = {nullptr, nullptr, nullptr};
+    void release()
+    {
+        for (auto &x : exec) {
+            if (x) cudaGraphExecDestroy(x);
+            x = nullptr;
+        }
+    }
+    MsResult() = default;
+    MsResult(const MsResult &) = delete;
+    MsResult &operator=(const MsResult &) = delete;
+    ~MsResult() { release(); }
 };
 
 void ms_layout(Carve &c, const Geom &g, int ns, const void *d_b, void *d_x, MsBuffers &w);
