@@ -67,22 +67,28 @@ __global__ void __launch_bounds__(256, MB) dslash_full_kernel(Geom g, int pv, Li
 // (half > 0: full-lattice fields, blockIdx.y = p), or sigma * pvec - D src when pvec is given.
 template <int LP, int SP, int S>
 __global__ void __launch_bounds__(S *split_sites(S)) dslash_split_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
-                                                                         const char *__restrict__ src,
-                                                                         const char *__restrict__ pvec,
-                                                                         char *__restrict__ dst, size_t half, int p,
-                                                                         double sigma, const int *__restrict__ gate)
+                                                                         const char *src, const char *pvec, char *dst,
+                                                                         size_t half, int p, double sigma,
+                                                                         const int *gate)
 {
-    if (gate && *gate == 0) return;
+    pdl_trigger();
     using T = typename Acc2<LP, SP>::T;
     constexpr int NS = split_sites(S);
     __shared__ T part[(S - 1) * 6 * NS];
     const int i = blockIdx.x * NS + threadIdx.x % NS;
     const int par = half ? (int)blockIdx.y : p;
     T acc[6];
-    if (!dslash_site_split<LP, SP, T, S>(g, pv, fat, lng, src + (1 - par) * half, par, i, i < g.vh, part, acc)) return;
+    bool on;
+    const auto ready = [&] {
+        pdl_wait();
+        return !gate || *gate != 0;
+    };
+    if (!dslash_site_split<LP, SP, T, S>(g, pv, fat, lng, src + (1 - par) * half, par, i, i < g.vh, part, acc, ready,
+                                         &on))
+        return;
     if (pvec) {
         T pv6[6];
-        ld_spinor<SP>(pvec + par * half, pv, i, pv6);
+        ld_spinor_coherent<SP>(pvec + par * half, pv, i, pv6);
 #pragma unroll
         for (int k = 0; k < 6; ++k) acc[k] = (T)sigma * pv6[k] - acc[k];
     }
@@ -128,9 +134,11 @@ static int threads_per_site(int lp, int sites)
         constexpr int MB = SiteCtas<LPv>::v; CALL;                  \
     }
 
+// follows: the launch before this one in the stream is a split kernel too (the first half of sigma - D D), and this one
+// may start beside its end
 template <int LP, int SP>
 static cudaError_t launch_split(int S, const Geom &g, const GaugeDev &gd, const void *src, const void *pvec, void *dst,
-                                size_t half, int p, double sigma, const int *gate, cudaStream_t s)
+                                size_t half, int p, double sigma, const int *gate, cudaStream_t s, bool follows = false)
 {
     const int ns = split_sites(S);
     const dim3 grid((g.vh + ns - 1) / ns, half ? 2 : 1);
@@ -138,13 +146,14 @@ static cudaError_t launch_split(int S, const Geom &g, const GaugeDev &gd, const 
     auto a = static_cast<const char *>(src);
     auto b = static_cast<const char *>(pvec);
     auto d = static_cast<char *>(dst);
-#define KQ_SPLIT(SV) \
-    dslash_split_kernel<LP, SP, SV><<<grid, bs, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], a, b, d, half, p, sigma, gate)
-    if (S == 2) KQ_SPLIT(2);
-    else if (S == 4) KQ_SPLIT(4);
-    else KQ_SPLIT(8);
-#undef KQ_SPLIT
-    return cudaGetLastError();
+    auto go = [&](auto kernel) -> cudaError_t {
+        if (follows)
+            return launch_pdl(kernel, grid, bs, s, g, pv, gd.fat[LP], gd.lng[LP], a, b, d, half, p, sigma, gate);
+        kernel<<<grid, bs, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], a, b, d, half, p, sigma, gate);
+        return cudaGetLastError();
+    };
+    return S == 2 ? go(dslash_split_kernel<LP, SP, 2>) : S == 4 ? go(dslash_split_kernel<LP, SP, 4>)
+                                                                 : go(dslash_split_kernel<LP, SP, 8>);
 }
 
 cudaError_t launch_dslash2(const Geom &g, const GaugeDev &gd, int lp, int sp, const void *src, void *dst,
@@ -198,7 +207,7 @@ cudaError_t launch_mdagm2(const Geom &g, const GaugeDev &gd, int lp, int sp, dou
     cudaError_t e = launch_dslash2(g, gd, lp, sp, src, tmp, 1 - parity, nullptr, s, 0);
     if (e != cudaSuccess) return e;
     if (const int S = threads_per_site(lp, g.vh); S > 1) {
-        KQ_DISPATCH_PAIR(lp, sp, e = (launch_split<LP, SP>(S, g, gd, tmp, src, dst, 0, parity, sigma, nullptr, s)));
+        KQ_DISPATCH_PAIR(lp, sp, e = (launch_split<LP, SP>(S, g, gd, tmp, src, dst, 0, parity, sigma, nullptr, s, true)));
         return e;
     }
     const int bs = 256;
@@ -226,7 +235,7 @@ cudaError_t launch_dslash_full(const Geom &g, const GaugeDev &gd, int prec, cons
     const size_t half = spinor_bytes(g, prec);
     if (const int S = threads_per_site(prec, 2 * g.vh); S > 1) {
         cudaError_t e = cudaSuccess;
-        KQ_DISPATCH_PAIR(prec, prec, e = (launch_split<LP, SP>(S, g, gd, src, pvec, dst, half, 0, sigma, nullptr, s)));
+        KQ_DISPATCH_PAIR(prec, prec, e = (launch_split<LP, SP>(S, g, gd, src, pvec, dst, half, 0, sigma, nullptr, s, pvec != nullptr)));
         return e;
     }
     const dim3 grid((g.vh + 255) / 256, 2);

@@ -260,40 +260,72 @@ __device__ __forceinline__ void dslash_hop_pair(const Geom &g, int pv, const Lin
     const int n1 = nbr_index(g, c, i, dir, sgn), n3 = nbr_index(g, c, i, dir, 3 * sgn);
     T u[18], v[6];
     ld_link_fold<LP>(fat_b, pv, dir, sgn > 0 ? i : n1, fat, u);
-    ld_spinor_as<SP>(src, pv, n1, v);
+    ld_spinor_coherent<SP>(src, pv, n1, v);
     if (sgn > 0) mv_add(u, v, acc);
     else mdv_sub(u, v, acc);
     ld_link_fold<LP>(lng_b, pv, dir, sgn > 0 ? i : n3, lng, u);
-    ld_spinor_as<SP>(src, pv, n3, v);
+    ld_spinor_coherent<SP>(src, pv, n3, v);
     fold_long_spinor<LP>(rl, v);
     if (sgn > 0) mv_add(u, v, acc);
     else mdv_sub(u, v, acc);
 }
 
+// Programmatic dependent launch: a kernel launched with cudaLaunchAttributeProgrammaticStreamSerialization may start
+// once every CTA of the kernel before it has called pdl_trigger (or ended); pdl_wait returns when that kernel is complete
+// and its writes are visible.  Both do nothing in kernels launched without the attribute.  What the kernel before wrote
+// is read with plain loads after the wait (ld_spinor_coherent), never through the read-only path, which assumes data
+// that no one writes while the kernel runs, nor through a __restrict__ pointer, which the compiler may send there.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // acc = (D src)(i) in the threads of sub 0, which return true if `valid` (the site exists); every thread of the CTA
-// calls this.  part: (S - 1) * 6 * NS values of shared memory.
-template <int LP, int SP, typename T, int S>
+// calls this.  part: (S - 1) * 6 * NS values of shared memory.  ready() is called by every thread once its first two
+// links are on their way and before any field is read; where it returns false (for the whole CTA) nothing is computed and
+// *on is false.  A kernel that waits there for the one before it (pdl_wait) has its launch, its index arithmetic and
+// these link loads overlap that kernel's end.
+template <int LP, int SP, typename T, int S, typename Ready>
 __device__ __forceinline__ bool dslash_site_split(const Geom &g, int pv, const LinkSet &fat, const LinkSet &lng,
-                                                  const void *src, int p, int i, bool valid, T *part, T acc[6])
+                                                  const void *src, int p, int i, bool valid, T *part, T acc[6],
+                                                  Ready ready, bool *on)
 {
     static_assert(S == 2 || S == 4 || S == 8, "threads per site");
     constexpr int NS = split_sites(S);
+    constexpr int ND = S == 2 ? 2 : 1;  // directions per thread
     const int sub = threadIdx.x / NS, s = threadIdx.x % NS;
 #pragma unroll
     for (int k = 0; k < 6; ++k) acc[k] = T(0);
+    const SiteCoord c = site_coord(g, valid ? i : 0, p);
+    const void *fat_p = p ? fat.par[1] : fat.par[0], *fat_q = p ? fat.par[0] : fat.par[1];
+    const void *lng_p = p ? lng.par[1] : lng.par[0], *lng_q = p ? lng.par[0] : lng.par[1];
+    const T rl = fold_scale_long<LP, T>(fat, lng);
+    const int dir0 = S == 8 ? sub >> 1 : ND * sub;
+    const bool fwd0 = S < 8 || !(sub & 1);
+    const int n1 = valid ? nbr_index(g, c, i, dir0, fwd0 ? 1 : -1) : 0;
+    const int n3 = valid ? nbr_index(g, c, i, dir0, fwd0 ? 3 : -3) : 0;
+    T u1[18], u3[18];
     if (valid) {
-        const SiteCoord c = site_coord(g, i, p);
-        const void *fat_p = p ? fat.par[1] : fat.par[0], *fat_q = p ? fat.par[0] : fat.par[1];
-        const void *lng_p = p ? lng.par[1] : lng.par[0], *lng_q = p ? lng.par[0] : lng.par[1];
-        const T rl = fold_scale_long<LP, T>(fat, lng);
-        constexpr int ND = S == 2 ? 2 : 1;  // directions per thread
+        ld_link_fold<LP>(fwd0 ? fat_p : fat_q, pv, dir0, fwd0 ? i : n1, fat, u1);
+        ld_link_fold<LP>(fwd0 ? lng_p : lng_q, pv, dir0, fwd0 ? i : n3, lng, u3);
+    }
+    *on = ready();
+    if (!*on) return false;
+    if (valid) {
+        T v[6], w[6];
+        ld_spinor_coherent<SP>(src, pv, n1, v);
+        ld_spinor_coherent<SP>(src, pv, n3, w);
+        fold_long_spinor<LP>(rl, w);
+        if (fwd0) {
+            mv_add(u1, v, acc);
+            mv_add(u3, w, acc);
+        } else {
+            mdv_sub(u1, v, acc);
+            mdv_sub(u3, w, acc);
+        }
+        if (S < 8) dslash_hop_pair<LP, SP, T>(g, pv, fat, lng, fat_q, lng_q, src, c, i, dir0, -1, rl, acc);
 #pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            const int dir = S == 8 ? sub >> 1 : ND * sub + d;
-            if (S < 8 || !(sub & 1))
-                dslash_hop_pair<LP, SP, T>(g, pv, fat, lng, fat_p, lng_p, src, c, i, dir, 1, rl, acc);
-            if (S < 8 || (sub & 1))
-                dslash_hop_pair<LP, SP, T>(g, pv, fat, lng, fat_q, lng_q, src, c, i, dir, -1, rl, acc);
+        for (int d = 1; d < ND; ++d) {
+            dslash_hop_pair<LP, SP, T>(g, pv, fat, lng, fat_p, lng_p, src, c, i, dir0 + d, 1, rl, acc);
+            dslash_hop_pair<LP, SP, T>(g, pv, fat, lng, fat_q, lng_q, src, c, i, dir0 + d, -1, rl, acc);
         }
     }
     if (sub) {
@@ -476,7 +508,7 @@ __device__ __forceinline__ double partials_sum(const double *partials, int n, do
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int b = b0 + u * (int)blockDim.x;
-            w[u] = b < n ? __ldcg(partials + b) : 0.0;
+            w[u] = b < n ? *((volatile const double *)partials + b) : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) s += w[u];

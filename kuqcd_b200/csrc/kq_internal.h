@@ -93,6 +93,23 @@ struct CgmState;
 cudaError_t launch_dslash_axmy_dot(const Geom &g, const GaugeDev &gd, int prec, const void *tmp, const void *p,
                                    void *s_out, int parity, CgmState *st, cudaStream_t s);
 
+// Launch with programmatic stream serialization: the kernel may start while the one before it in the stream ends (both
+// use pdl_trigger / pdl_wait of kq_dslash_core.cuh).
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int block, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // layout conversion (host records staged on the device, kuqcd.cpp:103-169 layouts)
 // `scratch` is one device word used for the HALF scale reduction.
 cudaError_t links_from_host_record(const Geom &g, const void *d_rec, int rec_prec, double factor, LinkSet &out,

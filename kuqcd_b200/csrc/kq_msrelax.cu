@@ -92,19 +92,25 @@ __global__ void __launch_bounds__(kBSm) ms_init_kernel(int vh, int pv, const voi
 __host__ __device__ constexpr int ms_threads(int S) { return S == 1 ? kBSm : S * split_sites(S); }
 __host__ __device__ constexpr int ms_sites(int S) { return S == 1 ? kBSm : split_sites(S); }
 
-// acc = (D src)(i) for this thread's output site i of parity p; false in threads without one
+// acc = (D src)(i) for this thread's output site i of parity p; false in threads without one.  *on: whether iterations
+// still run (`active`).  With S > 1 the kernel may have been started beside the end of the one before it.
 template <int LP, int SP, typename T, int S>
 __device__ __forceinline__ bool ms_site(const Geom &g, int pv, const LinkSet &fat, const LinkSet &lng, const void *src,
-                                        int p, int &i, T acc[6])
+                                        int p, const int *active, int &i, T acc[6], bool *on)
 {
     i = blockIdx.x * ms_sites(S) + threadIdx.x % ms_sites(S);
     if constexpr (S == 1) {
-        if (i >= g.vh) return false;
+        *on = *active != 0;
+        if (!*on || i >= g.vh) return false;
         dslash_site_t<LP, SP, T>(g, pv, fat, lng, src, p, i, acc);
         return true;
     } else {
+        const auto ready = [&] {
+            pdl_wait();
+            return *active != 0;
+        };
         __shared__ T part[(S - 1) * 6 * ms_sites(S)];
-        return dslash_site_split<LP, SP, T, S>(g, pv, fat, lng, src, p, i, i < g.vh, part, acc);
+        return dslash_site_split<LP, SP, T, S>(g, pv, fat, lng, src, p, i, i < g.vh, part, acc, ready, on);
     }
 }
 
@@ -113,16 +119,19 @@ __device__ __forceinline__ bool ms_site(const Geom &g, int pv, const LinkSet &fa
 // within its chunk.  S > 1: S threads per site (dslash_site_split).
 template <int LP, int SO, int S, int MB>
 __global__ void __launch_bounds__(ms_threads(S), MB) ms_dslash1_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
-                                                          const void *__restrict__ p0, void *__restrict__ tmp, int q,
-                                                          int slot, MsState *st, double *partials)
+                                                          const void *p0, void *tmp, int q, int slot, MsState *st,
+                                                          double *partials)
 {
-    if (st->active[slot] == 0) return;
+    pdl_trigger();
     __shared__ double sm[32];
     typedef typename Acc2<LP, LP>::T T;
     T acc[6];
     double tt = 0.0;
     int i;
-    if (ms_site<LP, 0, T, S>(g, pv, fat, lng, p0, q, i, acc)) {
+    bool on;
+    const bool mine = ms_site<LP, 0, T, S>(g, pv, fat, lng, p0, q, &st->active[slot], i, acc, &on);
+    if (!on) return;
+    if (mine) {
         st_spinor_as<SO>(tmp, pv, i, acc);
 #pragma unroll
         for (int k = 0; k < 6; ++k) tt += (double)acc[k] * (double)acc[k];
@@ -140,23 +149,25 @@ __global__ void __launch_bounds__(ms_threads(S), MB) ms_dslash1_kernel(Geom g, i
 // ring; |r|^2, then the alpha step
 template <int LP, int SI, int S, int MB>
 __global__ void __launch_bounds__(ms_threads(S), MB) ms_dslash2_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
-                                                          const void *__restrict__ tmp, const void *__restrict__ p0,
-                                                          char *ring, size_t vb, int p, int slot,
-                                                          MsState *st, double *partials)
+                                                          const void *tmp, const void *p0, char *ring, size_t vb,
+                                                          int p, int slot, MsState *st, double *partials)
 {
-    if (st->active[slot] == 0) return;
+    pdl_trigger();
     __shared__ double sm[32];
-    const int it = st->iter;  // iterations completed before this one
-    const char *rin = ring + (size_t)(it % kWin) * vb;
-    char *rout = ring + (size_t)((it + 1) % kWin) * vb;
     typedef typename Acc2<LP, LP>::T T;
     T acc[6];
     double nn = 0.0;
     int i;
-    if (ms_site<LP, SI, T, S>(g, pv, fat, lng, tmp, p, i, acc)) {
+    bool on;
+    const bool mine = ms_site<LP, SI, T, S>(g, pv, fat, lng, tmp, p, &st->active[slot], i, acc, &on);
+    if (!on) return;
+    if (mine) {
+        const int it = st->iter;  // iterations completed before this one
+        const char *rin = ring + (size_t)(it % kWin) * vb;
+        char *rout = ring + (size_t)((it + 1) % kWin) * vb;
         double pv6[6], rv[6];
-        ld_spinor<0>(p0, pv, i, pv6);
-        ld_spinor<0>(rin, pv, i, rv);
+        ld_spinor_coherent<0>(p0, pv, i, pv6);
+        ld_spinor_coherent<0>(rin, pv, i, rv);
         const double sig = st->shift[0], b0 = st->b0;
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
@@ -178,6 +189,8 @@ __global__ void __launch_bounds__(ms_threads(S), MB) ms_dslash2_kernel(Geom g, i
 __global__ void __launch_bounds__(kBSm) ms_p0_kernel(int vh, int pv, const char *ring, size_t vb, void *p0,
                                                      int slot, MsState *st)
 {
+    pdl_trigger();
+    pdl_wait();
     const bool on = st->active[slot] != 0;
     if (blockIdx.x == 0) {
         const bool go = on && ms_shift_step(st);
@@ -189,8 +202,8 @@ __global__ void __launch_bounds__(kBSm) ms_p0_kernel(int vh, int pv, const char 
     if (i >= vh) return;
     const char *r = ring + (size_t)(st->iter % kWin) * vb;
     double rv[6], pv6[6];
-    ld_spinor<0>(r, pv, i, rv);
-    ld_spinor<0>(p0, pv, i, pv6);
+    ld_spinor_coherent<0>(r, pv, i, rv);
+    ld_spinor_coherent<0>(p0, pv, i, pv6);
     const double a0 = st->a0;
 #pragma unroll
     for (int k = 0; k < 6; ++k) pv6[k] = rv[k] + a0 * pv6[k];
@@ -278,11 +291,18 @@ static int ms_split(int lp, int vh)
 template <int LP, int S, int MB>
 static void enqueue_ms_dslash(const Geom &g, const GaugeDev &gd, const MsBuffers &w, int parity, int it, cudaStream_t s)
 {
-    const int pv = pad_sites(g.vh), nb = (g.vh + ms_sites(S) - 1) / ms_sites(S);
-    ms_dslash1_kernel<LP, LP, S, MB><<<nb, ms_threads(S), 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.p0, w.tmp, 1 - parity,
-                                                              it & 1, w.st, w.partials);
-    ms_dslash2_kernel<LP, LP, S, MB><<<nb, ms_threads(S), 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.tmp, w.p0,
-                                                              (char *)w.ring, w.vb, parity, it & 1, w.st, w.partials);
+    const int pv = pad_sites(g.vh), nb = (g.vh + ms_sites(S) - 1) / ms_sites(S), nt = ms_threads(S);
+    if constexpr (S > 1) {
+        launch_pdl(ms_dslash1_kernel<LP, LP, S, MB>, nb, nt, s, g, pv, gd.fat[LP], gd.lng[LP], w.p0, w.tmp, 1 - parity,
+                   it & 1, w.st, w.partials);
+        launch_pdl(ms_dslash2_kernel<LP, LP, S, MB>, nb, nt, s, g, pv, gd.fat[LP], gd.lng[LP], w.tmp, w.p0, (char *)w.ring,
+                   w.vb, parity, it & 1, w.st, w.partials);
+    } else {
+        ms_dslash1_kernel<LP, LP, S, MB><<<nb, nt, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.p0, w.tmp, 1 - parity, it & 1,
+                                                           w.st, w.partials);
+        ms_dslash2_kernel<LP, LP, S, MB><<<nb, nt, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], w.tmp, w.p0, (char *)w.ring, w.vb,
+                                                           parity, it & 1, w.st, w.partials);
+    }
 }
 
 template <int LP>
@@ -290,8 +310,9 @@ static void enqueue_ms_chunk(const Geom &g, const GaugeDev &gd, const MsBuffers 
                              cudaStream_t s)
 {
     const int pv = pad_sites(g.vh), nb = (g.vh + kBSm - 1) / kBSm;
+    const int S = ms_split(LP, g.vh);
     for (int it = 0; it < kChunk; ++it) {
-        switch (ms_split(LP, g.vh)) {
+        switch (S) {
             case 8: enqueue_ms_dslash<LP, 8, 0>(g, gd, w, parity, it, s); break;
             case 4: enqueue_ms_dslash<LP, 4, 0>(g, gd, w, parity, it, s); break;
             case 2: enqueue_ms_dslash<LP, 2, 0>(g, gd, w, parity, it, s); break;
@@ -300,7 +321,8 @@ static void enqueue_ms_chunk(const Geom &g, const GaugeDev &gd, const MsBuffers 
                 else enqueue_ms_dslash<LP, 1, SiteCtas<LP>::v>(g, gd, w, parity, it, s);
                 break;
         }
-        ms_p0_kernel<<<nb + 1, kBSm, 0, s>>>(g.vh, pv, (const char *)w.ring, w.vb, w.p0, it & 1, w.st);
+        if (S > 1) launch_pdl(ms_p0_kernel, nb + 1, kBSm, s, g.vh, pv, (const char *)w.ring, w.vb, w.p0, it & 1, w.st);
+        else ms_p0_kernel<<<nb + 1, kBSm, 0, s>>>(g.vh, pv, (const char *)w.ring, w.vb, w.p0, it & 1, w.st);
     }
     switch (window_unroll()) {
         case 1: ms_window_kernel<1><<<nb, kBSm, 0, s>>>(g.vh, pv, (const char *)w.ring, w.vb, (char *)w.pw, (char *)w.x, w.st); break;

@@ -112,6 +112,28 @@ __device__ __forceinline__ void st_spinor_as(void *base, int pv, int i, const T 
     st_spinor<P>(base, pv, i, w);
 }
 
+// As ld_spinor_as, with plain loads (ld_spinor reads through the read-only path): for fields that a kernel still running
+// when this one starts may write (programmatic dependent launch).  `base` must not come from a __restrict__ pointer.
+template <int P, typename T>
+__device__ __forceinline__ void ld_spinor_coherent(const void *base, int pv, int i, T v[6])
+{
+    if constexpr (P == 0) {
+        const double2 *b = static_cast<const double2 *>(base);
+        const double2 a = b[i], c = b[pv + i], d = b[2 * pv + i];
+        v[0] = (T)a.x; v[1] = (T)a.y; v[2] = (T)c.x; v[3] = (T)c.y; v[4] = (T)d.x; v[5] = (T)d.y;
+    } else if constexpr (P == 1) {
+        const float4 a = static_cast<const float4 *>(base)[i];
+        const float2 c = reinterpret_cast<const float2 *>(static_cast<const float4 *>(base) + pv)[i];
+        v[0] = (T)a.x; v[1] = (T)a.y; v[2] = (T)a.z; v[3] = (T)a.w; v[4] = (T)c.x; v[5] = (T)c.y;
+    } else {
+        const int4 w = static_cast<const int4 *>(base)[i];
+        const float s = __int_as_float(w.w) * (1.0f / 32767.0f);
+        v[0] = (T)(lo16(w.x) * s); v[1] = (T)(hi16(w.x) * s);
+        v[2] = (T)(lo16(w.y) * s); v[3] = (T)(hi16(w.y) * s);
+        v[4] = (T)(lo16(w.z) * s); v[5] = (T)(hi16(w.z) * s);
+    }
+}
+
 // ------------------------------------------------------------------------------------------------ links
 // One 3x3 complex matrix, row-major u[2*(col + 3*row)] (re, im).
 // FP64: 9 double2 planes per direction.     dir stride = 9 * pv double2
