@@ -278,12 +278,12 @@ static int window_unroll()
 }
 
 // ---------------------------------------------------------------------------------------------------- driver
-// Threads per site of the dslash steps.  The FP64 and FP32 ones gain as the stand-alone kernels do (16^4: FP64 18.5
-// us with one thread per site and 14.4 with two, FP32 14.0 and, with four, 9.3 us); the HALF ones, short beside their
-// reduction, only on smaller lattices (12^4: 8.9 and, with four, 7.3 us; 16^4: 9.5 us with one thread, 9.6 with two).
+// Threads per site of the dslash steps, by the limits of the stand-alone kernels.  (With the launches overlapped, 16^4
+// and twelve shifts: FP64 with two threads per site 12.5 ms, with four 14.3 ms; the mixed solve with the HALF steps at
+// one thread per site 10.76 ms, at four 10.59 ms.)
 static int ms_split(int lp, int vh)
 {
-    return split_of(vh, lp == P64 ? kSplitLimit64 : lp == P32 ? kSplitLimit32 : 65000);
+    return split_of(vh, lp == P64 ? kSplitLimit64 : lp == P32 ? kSplitLimit32 : kSplitLimit16);
 }
 
 // MB: resident CTAs per SM the kernels are compiled for (0: no bound, best for S > 1: at one the compiler takes 112
