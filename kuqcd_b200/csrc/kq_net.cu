@@ -321,7 +321,10 @@ KQ_API KuQCDStatus kq_net_train_pair(kq_net *n, const void *d_r, const void *d_e
     cudaError_t e = forward(n, d_r, parity, 1.0);
     double l = 0;
     int cur = 0;
-    if (e == cudaSuccess) e = ptc_loss(ctx->g, n->cact[0], d_e, parity, 1.0 / e_norm2, n->gbuf[cur], n->lpart, &l, s);
+    // the loss stays on the device until the whole pair is enqueued: read in the middle it left the GPU idle for as
+    // long as the host took to enqueue the backward pass
+    double *d_loss = n->lpart + (ctx->g.vh + 255) / 256;
+    if (e == cudaSuccess) e = ptc_loss(ctx->g, n->cact[0], d_e, parity, 1.0 / e_norm2, n->gbuf[cur], n->lpart, d_loss, s);
     auto accum = [&](int layer, bool adjoint) {
         if (e != cudaSuccess) return;
         const int ci = n->ch[layer], co = n->ch[layer + 1];
@@ -349,6 +352,7 @@ KQ_API KuQCDStatus kq_net_train_pair(kq_net *n, const void *d_r, const void *d_e
             cur = 1 - cur;
         }
     }
+    if (e == cudaSuccess && loss) e = cudaMemcpyAsync(&l, d_loss, sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = ptc_check_fault(s);
     if (loss) *loss = l;
     if (e != cudaSuccess) set_last_error(std::string("kq_net_train_pair: ") + net_error_text(e));

@@ -36,6 +36,7 @@ namespace kq {
 constexpr int kTile = 128;  // sites per CTA
 constexpr int kThr = 128;   // threads per CTA (4 warps)
 constexpr int kPaths = 9;
+constexpr int kNT = 16;                      // N of the tensor-core tile (C_out * 2 padded)
 
 __host__ __device__ constexpr int kpad_of(int cin) { return ((cin * kPaths * 2 + 15) / 16) * 16; }
 __host__ __device__ constexpr int npad_of(int cout) { return ((cout * 2 + 7) / 8) * 8; }
@@ -50,6 +51,20 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 __device__ __forceinline__ float2 ld_act(const float2 *act, int pv, int c, int par, int a, int i)
 {
     return __ldg(act + (size_t)((c * 2 + par) * 3 + a) * pv + i);
+}
+
+// the B operand [kNT x KP] from the layer's [NP][KP] matrix, 16 bytes (8 columns of a row: one row of a core matrix) at
+// a time; rows past NP are zero
+template <int KP, int NP>
+__device__ __forceinline__ void load_b(unsigned char *Bs, const __nv_bfloat16 *__restrict__ Bt, int t, int threads)
+{
+    static_assert(KP % 8 == 0, "whole 16-byte rows");
+    const uint4 *src = reinterpret_cast<const uint4 *>(Bt);
+    for (int e = t; e < kNT * (KP / 8); e += threads) {
+        const int n = e / (KP / 8), k8 = e - n * (KP / 8);
+        *reinterpret_cast<uint4 *>(Bs + umma::kmajor_offset(n, 8 * k8, KP)) =
+            n < NP ? __ldg(src + n * (KP / 8) + k8) : make_uint4(0, 0, 0, 0);
+    }
 }
 
 // Gather the transported inputs of site i (parity par) path by path: emit(p, vals) with vals[a][2 c + reim] the
@@ -159,7 +174,6 @@ __device__ __forceinline__ void gather_tile(const Geom &g, int pv, const LinkSet
 
 // out (C_out channels, both parities) = layer(in); Bt: [NP][KP] BF16 weights (device), built by the host.
 // fault: set when the tensor cores did not signal completion within the wait limit (the tile is then not written).
-constexpr int kNT = 16;                      // N of the tensor-core tile (C_out * 2 padded)
 constexpr uint32_t kTmemCols = 64;           // 3 colours x 16 FP32 accumulator columns, rounded up
 constexpr uint32_t kWaitLimit = 1u << 24;    // mbarrier polls before a tile gives up
 
@@ -238,14 +252,19 @@ __global__ void __launch_bounds__(kThr) ptc_forward_kernel(Geom g, int pv, LinkS
 // Forward layer with 8 input channels, K-chunked by path: K = 9 paths x 16 columns, and each path's 16 columns of
 // the gathered tile are one K = 16 step of the MMA.  The CTA gathers path j into one of two chunk buffers while the
 // tensor cores multiply chunk j - 1 from the other, so shared memory holds 2 x 3 x [128 x 16] BF16 (24 KB) instead
-// of the whole [128 x 144] tile per colour (108 KB): five or more CTAs fit on an SM and hide each other's gather
-// latency.  Chunk j's MMAs commit to mbarrier (j & 1); before chunk j + 2 overwrites that buffer every thread waits
-// for the commit's phase (j >> 1) & 1 (bounded, as in the whole-tile kernel).
+// of the whole [128 x 144] tile per colour (108 KB).  Chunk j's MMAs commit to mbarrier (j & 1); before chunk j + 2
+// overwrites that buffer every thread waits for the commit's phase (j >> 1) & 1 (bounded, as in the whole-tile kernel).
+// The layer is bound by the latency of the gather, 24 scattered 8-byte loads per site and path: the loads of path j + 1
+// are issued once path j's values are used, ahead of its barriers.  32^4, 8 -> 8 channels: 356 us with four CTAs per SM
+// at 128 registers; without the early loads 450 us with six at 80.  One application of M: 1.23 ms (1.50 ms before); with
+// two or four threads per site, each loading the links again, 1.38 and 1.78 ms; with the next loads issued channel by
+// channel among the mat-vecs 1.43 ms.
 constexpr uint32_t kChunkColBytes = kTile * 16 * 2;  // one colour's [128 x 16] BF16 chunk
-template <int COUT, int MINB>
-__global__ void __launch_bounds__(kThr, MINB) ptc_forward8_kernel(Geom g, int pv, LinkSet fat, const float2 *__restrict__ in,
-                                                            float2 *__restrict__ out, const __nv_bfloat16 *__restrict__ Bt,
-                                                            int swap_paths, int *fault)
+template <int COUT>
+__global__ void __launch_bounds__(kThr, 4) ptc_forward8_kernel(Geom g, int pv, LinkSet fat, const float2 *__restrict__ in,
+                                                               float2 *__restrict__ out,
+                                                               const __nv_bfloat16 *__restrict__ Bt, int swap_paths,
+                                                               int *fault)
 {
     constexpr int CIN = 8, KP = kpad_of(CIN), NP = npad_of(COUT);
     constexpr uint32_t CH_BYTES = 3 * kChunkColBytes;  // one chunk: 3 colours
@@ -265,91 +284,75 @@ __global__ void __launch_bounds__(kThr, MINB) ptc_forward8_kernel(Geom g, int pv
         umma::mbar_init(&mbar[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int e = t; e < kNT * KP; e += kThr) {
-        const int n = e / KP, k = e - n * KP;
-        *reinterpret_cast<__nv_bfloat16 *>(Bs + umma::kmajor_offset(n, k, KP)) =
-            n < NP ? Bt[n * KP + k] : __float2bfloat16_rn(0.f);
-    }
-    umma::fence_before_sync();
-    __syncthreads();
-    umma::fence_after_sync();
-    const uint32_t tbase = *tslot;
     const int i = base + t;
     const bool valid = i < g.vh;
     const SiteCoord cd = site_coord(g, valid ? i : 0, par);
     const int q = 1 - par;
     const void *fat_p = par ? fat.par[1] : fat.par[0];
     const void *fat_q = par ? fat.par[0] : fat.par[1];
+    // path j: identity (j = 0), then for each direction the forward and the backward hop
+    float u[18], v[CIN][6];
+    auto load = [&](int j) {
+        const int n = j == 0 ? i : nbr_index(g, cd, i, (j - 1) >> 1, (j & 1) ? 1 : -1);
+        if (j > 0) ld_link<1>((j & 1) ? fat_p : fat_q, pv, (j - 1) >> 1, (j & 1) ? i : n, 1.f, u);
+#pragma unroll
+        for (int c = 0; c < CIN; ++c)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float2 w = ld_act(in, pv, c, j == 0 ? par : q, a, n);
+                v[c][2 * a] = w.x;
+                v[c][2 * a + 1] = w.y;
+            }
+    };
+    if (valid) load(0);
+    load_b<KP, NP>(Bs, Bt, t, kThr);
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tbase = *tslot;
     constexpr uint32_t idesc = umma::idesc_bf16_f32(kTile, kNT);
     const uint32_t a0 = umma::smem_u32(Ach), b0 = umma::smem_u32(Bs);
     bool ok = true;
 #pragma unroll 1
     for (int j = 0; j < kPaths && ok; ++j) {
         const int buf = j & 1;
+        const int dir = (j - 1) >> 1, fb = (j - 1) & 1;
+        const int p = j == 0 ? 0 : 1 + 2 * dir + (swap_paths ? 1 - fb : fb);
+        uint32_t w[3][CIN];  // (re, im) of each colour and channel as a BF16 pair
+        if (valid) {
+#pragma unroll
+            for (int c = 0; c < CIN; ++c) {
+                float o[6] = {0, 0, 0, 0, 0, 0};
+                if (j == 0) {
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) o[k] = v[c][k];
+                } else if (fb == 0) {
+                    mv_add(u, v[c], o);
+                } else {
+                    mdv_sub(u, v[c], o);
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) o[k] = -o[k];
+                }
+#pragma unroll
+                for (int a = 0; a < 3; ++a) w[a][c] = pack_bf16(o[2 * a], o[2 * a + 1]);
+            }
+            if (j + 1 < kPaths) load(j + 1);
+        } else {
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int c = 0; c < CIN; ++c) w[a][c] = 0u;
+        }
         if (j >= 2) {  // the MMAs of chunk j - 2 must be done reading this buffer
             ok = __syncthreads_and(umma::mbar_wait(&mbar[buf], ((j - 2) >> 1) & 1, kWaitLimit));
             if (!ok) break;
             umma::fence_after_sync();
         }
-        // path j: identity, then for each direction the forward and the backward hop
-        int p = 0;
-        float vals[3][2 * CIN];
-        if (j == 0) {
-#pragma unroll
-            for (int c = 0; c < CIN; ++c)
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const float2 v = valid ? ld_act(in, pv, c, par, a, i) : make_float2(0.f, 0.f);
-                    vals[a][2 * c] = v.x;
-                    vals[a][2 * c + 1] = v.y;
-                }
-        } else {
-            const int dir = (j - 1) >> 1, fb = (j - 1) & 1;
-            p = 1 + 2 * dir + (swap_paths ? 1 - fb : fb);
-            if (valid) {
-                const int nb = nbr_index(g, cd, i, dir, fb == 0 ? 1 : -1);
-                float u[18];
-                ld_link<1>(fb == 0 ? fat_p : fat_q, pv, dir, fb == 0 ? i : nb, 1.f, u);
-#pragma unroll
-                for (int c = 0; c < CIN; ++c) {
-                    float v[6], o[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const float2 w = ld_act(in, pv, c, q, a, nb);
-                        v[2 * a] = w.x;
-                        v[2 * a + 1] = w.y;
-                    }
-                    if (fb == 0) mv_add(u, v, o);
-                    else {
-                        mdv_sub(u, v, o);
-#pragma unroll
-                        for (int k = 0; k < 6; ++k) o[k] = -o[k];
-                    }
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        vals[a][2 * c] = o[2 * a];
-                        vals[a][2 * c + 1] = o[2 * a + 1];
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int k = 0; k < 2 * CIN; ++k) vals[a][k] = 0.f;
-            }
-        }
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            unsigned char *col = Ach + buf * CH_BYTES + a * kChunkColBytes;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint4 w;
-                w.x = pack_bf16(vals[a][8 * h + 0], vals[a][8 * h + 1]);
-                w.y = pack_bf16(vals[a][8 * h + 2], vals[a][8 * h + 3]);
-                w.z = pack_bf16(vals[a][8 * h + 4], vals[a][8 * h + 5]);
-                w.w = pack_bf16(vals[a][8 * h + 6], vals[a][8 * h + 7]);
-                *reinterpret_cast<uint4 *>(col + umma::kmajor_offset(t, 8 * h, 16)) = w;
-            }
+            unsigned char *col = Ach + buf * CH_BYTES + a * kChunkColBytes + umma::kmajor_offset(t, 0, 16);
+            *reinterpret_cast<uint4 *>(col) = make_uint4(w[a][0], w[a][1], w[a][2], w[a][3]);
+            *reinterpret_cast<uint4 *>(col + 128) = make_uint4(w[a][4], w[a][5], w[a][6], w[a][7]);
         }
         umma::fence_smem_to_async();
         umma::fence_before_sync();
@@ -389,14 +392,99 @@ __global__ void __launch_bounds__(kThr, MINB) ptc_forward8_kernel(Geom g, int pv
     if (warp == 0) umma::tmem_dealloc(tbase, kTmemCols);
 }
 
-// ---------------------------------------------------------------------------------------------------- weight grad
+// gather_tile<8> with four threads per site, one direction each: thread t of the CTA takes site base + t % 128, the
+// forward and the backward hop of direction t / 128 in all channels (so every link is loaded once), and two channels of
+// the identity path.  All loads of a hop are in flight together, the backward hop's behind the forward hop's values.
+__device__ __forceinline__ void gather_tile8(const Geom &g, int pv, const LinkSet &fat, const float2 *in, int par, int base,
+                                             int t, bool swap_paths, unsigned char *As)
+{
+    constexpr int KP = kpad_of(8);
+    constexpr uint32_t A_BYTES = kTile * KP * 2;
+    const int row = t % kTile, dir = t / kTile, i = base + row;
+    auto store = [&](int p, const uint32_t (&w)[3][8]) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            unsigned char *d = As + a * A_BYTES + umma::kmajor_offset(row, p * 16, KP);
+            *reinterpret_cast<uint4 *>(d) = make_uint4(w[a][0], w[a][1], w[a][2], w[a][3]);
+            *reinterpret_cast<uint4 *>(d + 128) = make_uint4(w[a][4], w[a][5], w[a][6], w[a][7]);
+        }
+    };
+    uint32_t w[3][8];
+    uint2 own[3];
+    const bool valid = i < g.vh;
+    if (valid) {
+        const SiteCoord cd = site_coord(g, i, par);
+        const void *fat_p = par ? fat.par[1] : fat.par[0], *fat_q = par ? fat.par[0] : fat.par[1];
+        float u[18], v[8][6];
+        float2 id[3][2];
+        auto load = [&](int fb) {
+            const int n = nbr_index(g, cd, i, dir, fb == 0 ? 1 : -1);
+            ld_link<1>(fb == 0 ? fat_p : fat_q, pv, dir, fb == 0 ? i : n, 1.f, u);
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const float2 x = ld_act(in, pv, c, 1 - par, a, n);
+                    v[c][2 * a] = x.x;
+                    v[c][2 * a + 1] = x.y;
+                }
+        };
+        auto pack = [&](bool bwd) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                float o[6] = {0, 0, 0, 0, 0, 0};
+                if (!bwd) {
+                    mv_add(u, v[c], o);
+                } else {
+                    mdv_sub(u, v[c], o);
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) o[k] = -o[k];
+                }
+#pragma unroll
+                for (int a = 0; a < 3; ++a) w[a][c] = pack_bf16(o[2 * a], o[2 * a + 1]);
+            }
+        };
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) id[a][c] = ld_act(in, pv, 2 * dir + c, par, a, i);
+        load(0);
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            own[a] = make_uint2(pack_bf16(id[a][0].x, id[a][0].y), pack_bf16(id[a][1].x, id[a][1].y));
+        pack(false);
+        load(1);
+        store(1 + 2 * dir + (swap_paths ? 1 : 0), w);
+        pack(true);
+        store(1 + 2 * dir + (swap_paths ? 0 : 1), w);
+    } else {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            own[a] = make_uint2(0, 0);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) w[a][c] = 0u;
+        }
+        store(1 + 2 * dir, w);
+        store(2 + 2 * dir, w);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        *reinterpret_cast<uint2 *>(As + a * A_BYTES + umma::kmajor_offset(row, 4 * dir, KP)) = own[a];
+}
+
+constexpr int wgrad_threads(int cin) { return cin == 8 ? 4 * kThr : kThr; }
+
 // partial[cta][k][n] = sum over the tiles this CTA visits (tile = blockIdx.x + j * gridDim.x) and over their rows
 // (sites x colours) of T[row][k] * G[row][n]  (swap_paths: T gathered as by the adjoint layer).
+// With 8 input channels the tile's operands take most of an SM's shared memory, so one CTA runs per SM, and four threads
+// share a site (one direction each, gather_tile8) to keep the gather's loads in flight (16^4, 8 -> 8 channels: 50 us with
+// one thread per site, 42 with four).  With one input channel four CTAs of one thread per site fit an SM (47 us with one
+// CTA per SM, 18 with four).
 // Persistent: the accumulator D (M = k, N = 16) stays in tensor memory across all of the CTA's tiles.  A is the
 // gathered tile read MN-major (M = k, K = sites); B = G, [site][n] in 8 x 16-byte core matrices, also MN-major.
 // With KP = 144 two M tiles cover k < 256; the rows of D past KP read neighbouring data and are never stored.
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kThr) ptc_wgrad_kernel(Geom g, int pv, LinkSet fat, const float2 *__restrict__ in,
+__global__ void __launch_bounds__(wgrad_threads(CIN)) ptc_wgrad_kernel(Geom g, int pv, LinkSet fat, const float2 *__restrict__ in,
                                                          const float2 *__restrict__ gout, float *__restrict__ partial,
                                                          int swap_paths, int *fault)
 {
@@ -430,28 +518,25 @@ __global__ void __launch_bounds__(kThr) ptc_wgrad_kernel(Geom g, int pv, LinkSet
         }
         const int par = tile & 1;  // parity-interleaved tile order, as in the forward kernels
         const int base = (tile >> 1) * kTile;
-        gather_tile<CIN>(g, pv, fat, in, par, base, t, swap_paths != 0, As);
-        const int i = base + t;
+        // the output gradient's rows, one colour per group of 128 threads where there are several
+        constexpr int PARTS = wgrad_threads(CIN) / kTile;
+        const int row = t % kTile, i = base + row;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            float gv[kNT];
+        for (int a = t / kTile; a < 3; a += PARTS) {
+            uint32_t gv[kNT / 2];
 #pragma unroll
             for (int o = 0; o < kNT / 2; ++o) {
                 float2 w = make_float2(0.f, 0.f);
                 if (o < COUT && i < g.vh) w = ld_act(gout, pv, o, par, a, i);
-                gv[2 * o] = w.x;
-                gv[2 * o + 1] = w.y;
+                gv[o] = pack_bf16(w.x, w.y);
             }
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint4 w;
-                w.x = pack_bf16(gv[8 * h + 0], gv[8 * h + 1]);
-                w.y = pack_bf16(gv[8 * h + 2], gv[8 * h + 3]);
-                w.z = pack_bf16(gv[8 * h + 4], gv[8 * h + 5]);
-                w.w = pack_bf16(gv[8 * h + 6], gv[8 * h + 7]);
-                *reinterpret_cast<uint4 *>(Gs + a * G_BYTES + (t >> 3) * G_GROUP + h * 128 + (t & 7) * 16) = w;
-            }
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<uint4 *>(Gs + a * G_BYTES + (row >> 3) * G_GROUP + h * 128 + (row & 7) * 16) =
+                    make_uint4(gv[4 * h], gv[4 * h + 1], gv[4 * h + 2], gv[4 * h + 3]);
         }
+        if constexpr (CIN == 8) gather_tile8(g, pv, fat, in, par, base, t, swap_paths != 0, As);
+        else gather_tile<CIN>(g, pv, fat, in, par, base, t, swap_paths != 0, As);
         umma::fence_smem_to_async();
         umma::fence_before_sync();
         __syncthreads();
@@ -479,7 +564,7 @@ __global__ void __launch_bounds__(kThr) ptc_wgrad_kernel(Geom g, int pv, LinkSet
     }
     umma::fence_after_sync();
     float *out = partial + (size_t)blockIdx.x * KP * NP;
-    if (ok) {
+    if (ok && warp < 4) {
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
             float d[16];
@@ -565,6 +650,14 @@ __global__ void ptc_loss_kernel(int vh, int pv, const float2 *__restrict__ y, co
     if (threadIdx.x == 0) partials[blockIdx.x] = l;
 }
 
+// *loss = sum of the loss kernel's partials, in a fixed order
+__global__ void __launch_bounds__(256) ptc_loss_sum_kernel(const double *partials, int n, double *loss)
+{
+    __shared__ double sm[32];
+    const double l = partials_sum(partials, n, sm);
+    if (threadIdx.x == 0) *loss = l;
+}
+
 // Adam on grad * grad_scale (the accumulated gradient of a batch times 1/batch); the accumulator is cleared here, so
 // the next batch starts from zero without a separate memset
 __global__ void ptc_adam_kernel(float *w, float *grad, float *m, float *v, int n, float lr, float grad_scale, float b1,
@@ -628,44 +721,18 @@ cudaError_t ptc_raise_fault_for_test()
     return cudaMemcpy(f, &one, sizeof(int), cudaMemcpyHostToDevice);
 }
 
-// Resident CTAs per SM the 8-channel kernel is compiled for (KUQCD_PTC_CTAS = 4 .. 7; 64 TMEM columns and 29 KB of
-// shared memory each, so 7 fit the SM's 512 columns and 228 KB).  The gather is latency-bound: six CTAs at 80
-// registers (8 B spilled) apply M in 1.50 ms at 32^4 against 1.79 ms for four at 128.
-static int ptc_ctas()
-{
-    static const int k = [] {
-        const char *e = getenv("KUQCD_PTC_CTAS");
-        const int v = e ? atoi(e) : 6;
-        return v >= 4 && v <= 7 ? v : 6;
-    }();
-    return k;
-}
-
-template <int COUT, int MINB>
-static cudaError_t run_forward8_b(const Geom &g, const LinkSet &fat, const float2 *in, float2 *out,
-                                  const __nv_bfloat16 *Bt, bool swap, cudaStream_t s)
-{
-    const int pv = pad_sites(g.vh);
-    const int tiles = 2 * ((g.vh + kTile - 1) / kTile);
-    const size_t sm = (size_t)2 * 3 * kChunkColBytes + (size_t)kNT * kpad_of(8) * 2 + 32;
-    KQ_CUDA_TRY(cudaFuncSetAttribute(ptc_forward8_kernel<COUT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sm));
-    int *fault = fault_flag();
-    if (!fault) return cudaErrorInvalidDevicePointer;
-    ptc_forward8_kernel<COUT, MINB><<<tiles, kThr, sm, s>>>(g, pv, fat, in, out, Bt, swap ? 1 : 0, fault);
-    return cudaGetLastError();
-}
-
 template <int COUT>
 static cudaError_t run_forward8(const Geom &g, const LinkSet &fat, const float2 *in, float2 *out,
                                 const __nv_bfloat16 *Bt, bool swap, cudaStream_t s)
 {
-    switch (ptc_ctas()) {
-        case 4: return run_forward8_b<COUT, 4>(g, fat, in, out, Bt, swap, s);
-        case 5: return run_forward8_b<COUT, 5>(g, fat, in, out, Bt, swap, s);
-        case 7: return run_forward8_b<COUT, 7>(g, fat, in, out, Bt, swap, s);
-        default: return run_forward8_b<COUT, 6>(g, fat, in, out, Bt, swap, s);
-    }
+    const int pv = pad_sites(g.vh);
+    const int tiles = 2 * ((g.vh + kTile - 1) / kTile);
+    const size_t sm = (size_t)2 * 3 * kChunkColBytes + (size_t)kNT * kpad_of(8) * 2 + 32;
+    KQ_CUDA_TRY(cudaFuncSetAttribute(ptc_forward8_kernel<COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    int *fault = fault_flag();
+    if (!fault) return cudaErrorInvalidDevicePointer;
+    ptc_forward8_kernel<COUT><<<tiles, kThr, sm, s>>>(g, pv, fat, in, out, Bt, swap ? 1 : 0, fault);
+    return cudaGetLastError();
 }
 
 template <int CIN, int COUT>
@@ -694,12 +761,13 @@ static cudaError_t run_wgrad(const Geom &g, const LinkSet &fat, const float2 *in
                                      (int)sm));
     int *fault = fault_flag();
     if (!fault) return cudaErrorInvalidDevicePointer;
-    // persistent: one CTA per SM (the operand tiles fill most of shared memory), each accumulating its tiles
+    // persistent, each CTA accumulating its tiles: one CTA per SM where the operand tiles fill most of shared memory,
+    // four where they take 45 KB
     int dev = 0, nsm = 148;
     KQ_CUDA_TRY(cudaGetDevice(&dev));
     KQ_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const int ctas = std::max(1, std::min(tiles, nsm));
-    ptc_wgrad_kernel<CIN, COUT><<<ctas, kThr, sm, s>>>(g, pv, fat, in, gout, partial, swap ? 1 : 0, fault);
+    const int ctas = std::max(1, std::min(tiles, CIN == 1 ? 4 * nsm : nsm));
+    ptc_wgrad_kernel<CIN, COUT><<<ctas, wgrad_threads(CIN), sm, s>>>(g, pv, fat, in, gout, partial, swap ? 1 : 0, fault);
     const int nelem = kpad_of(CIN) * npad_of(COUT);
     ptc_reduce_kernel<<<std::min(nelem, 1024), 256, 0, s>>>(partial, ctas, nelem, dB);
     return cudaGetLastError();
@@ -749,20 +817,12 @@ cudaError_t ptc_extract(const Geom &g, const float2 *act, int parity, void *dst,
 }
 
 cudaError_t ptc_loss(const Geom &g, const float2 *y, const void *e, int parity, double inv_e2, float2 *gout,
-                     double *partials, double *loss_host, cudaStream_t s)
+                     double *partials, double *loss, cudaStream_t s)
 {
     const int nb = (g.vh + 255) / 256;
     ptc_loss_kernel<<<nb, 256, 0, s>>>(g.vh, pad_sites(g.vh), y, e, parity, inv_e2, gout, partials);
-    KQ_CUDA_TRY(cudaGetLastError());
-    if (loss_host) {
-        std::vector<double> h(nb);
-        KQ_CUDA_TRY(cudaMemcpyAsync(h.data(), partials, sizeof(double) * nb, cudaMemcpyDeviceToHost, s));
-        KQ_CUDA_TRY(cudaStreamSynchronize(s));
-        double l = 0;
-        for (double v : h) l += v;
-        *loss_host = l;
-    }
-    return cudaSuccess;
+    ptc_loss_sum_kernel<<<1, 256, 0, s>>>(partials, nb, loss);
+    return cudaGetLastError();
 }
 
 cudaError_t ptc_adam(float *w, float *grad, float *m, float *v, int n, float lr, float grad_scale, int step,

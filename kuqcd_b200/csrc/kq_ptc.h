@@ -24,8 +24,9 @@ int ptc_tiles(const Geom &g);
 
 cudaError_t ptc_embed(const Geom &g, const void *src, int parity, float2 *act, double scale, cudaStream_t s);
 cudaError_t ptc_extract(const Geom &g, const float2 *act, int parity, void *dst, double scale, cudaStream_t s);
+// loss (device word): |y - e|^2 * inv_e2 on the parity sites
 cudaError_t ptc_loss(const Geom &g, const float2 *y, const void *e, int parity, double inv_e2, float2 *gout,
-                     double *partials, double *loss_host, cudaStream_t s);
+                     double *partials, double *loss, cudaStream_t s);
 // Adam step on grad * grad_scale; clears grad
 cudaError_t ptc_adam(float *w, float *grad, float *m, float *v, int n, float lr, float grad_scale, int step,
                      cudaStream_t s);
