@@ -95,12 +95,12 @@ __device__ __forceinline__ int tile_site(int tile, int spt, int s)
 
 // members of group G whose system iterates with operator precision M in this launch (uniform over the CTA: the
 // states only change in the scalar steps, which run after every tile of the system has passed)
-template <int R, int M>
+template <int M>
 __device__ __forceinline__ unsigned group_mask(const GroupDesc &G)
 {
     unsigned use = 0;
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+    for (int r = 0; r < kMaxR; ++r)
         if (r < G.n) {
             const MsState *st = c_sys[G.mem[r]].st;
             if (st->active[0] && st->mode == M) use |= 1u << r;
@@ -114,16 +114,16 @@ __device__ __forceinline__ unsigned group_mask(const GroupDesc &G)
 // link element is duplicated into both halves once per link (negated for the backward hops, so that one accumulator
 // takes all sixteen terms), and each packed FMA serves two members: 36 f32x2 FMAs per pair and link instead of 72.
 // Same terms in the same order as dslash_site_mrhs_t; a member outside `use` enters as zeros.
-template <int SP>
+template <int SP, bool ALL>
 __device__ __forceinline__ void ld_member_pair(const char *src0, size_t stride, int r0, unsigned use, int pv, int n,
                                                h2::f2 v[6])
 {
     float a[6], b[6];
-    if (use & (1u << r0)) ld_spinor_as<SP>(src0 + (size_t)r0 * stride, pv, n, a);
+    if (ALL || (use & (1u << r0))) ld_spinor_as<SP>(src0 + (size_t)r0 * stride, pv, n, a);
     else
 #pragma unroll
         for (int k = 0; k < 6; ++k) a[k] = 0.f;
-    if (use & (2u << r0)) ld_spinor_as<SP>(src0 + (size_t)(r0 + 1) * stride, pv, n, b);
+    if (ALL || (use & (2u << r0))) ld_spinor_as<SP>(src0 + (size_t)(r0 + 1) * stride, pv, n, b);
     else
 #pragma unroll
         for (int k = 0; k < 6; ++k) b[k] = 0.f;
@@ -131,7 +131,7 @@ __device__ __forceinline__ void ld_member_pair(const char *src0, size_t stride, 
     for (int k = 0; k < 6; ++k) v[k] = h2::pack(a[k], b[k]);
 }
 
-template <int LP, int SP, int RP>
+template <int LP, int SP, int RP, bool ALL>
 __device__ __forceinline__ void dslash_site_mrhs_pair(const Geom &g, int pv, const LinkSet &fat, const LinkSet &lng,
                                                       const char *src0, size_t stride, unsigned use, int p, int i,
                                                       float acc[RP][6])
@@ -163,9 +163,9 @@ __device__ __forceinline__ void dslash_site_mrhs_pair(const Geom &g, int pv, con
             for (int k = 0; k < 18; ++k) uu[k] = bwd ? pack(-u[k], -u[k]) : pack(u[k], u[k]);
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
-                if (!(use & (3u << (2 * q)))) continue;
+                if (!ALL && !(use & (3u << (2 * q)))) continue;
                 f2 v[6], w[3];
-                ld_member_pair<SP>(src0, stride, 2 * q, use, pv, n, v);
+                ld_member_pair<SP, ALL>(src0, stride, 2 * q, use, pv, n, v);
                 if (LP == 2 && isl)
 #pragma unroll
                     for (int k = 0; k < 6; ++k) v[k] = mul2(v[k], rl2);
@@ -188,20 +188,31 @@ __device__ __forceinline__ void dslash_site_mrhs_pair(const Geom &g, int pv, con
         }
 }
 
-// the grouped dslash of one site: FP32 arithmetic with an even member count in the packed member-pair form
+// The grouped dslash of one site: FP32 arithmetic with an even member count in the packed member-pair form.  Where every
+// member of the pass is applied -- members of one gauge field, mass and target change precision within a few iterations
+// of each other -- no test stands between the members' loads: with the tests the compiler loads one member's spinor,
+// waits, multiplies, and only then loads the next (FP64, four members at 24^3 x 48: half again the time).
+template <int M, int SP, typename T, int RP, bool ALL>
+__device__ __forceinline__ void grouped_site_of(const Geom &g, int pv, const LinkSet &fat, const LinkSet &lng,
+                                                const char *src0, size_t stride, unsigned use, int p, int i, T acc[RP][6])
+{
+    if constexpr (M != 0 && RP % 2 == 0)
+        dslash_site_mrhs_pair<M, SP, RP, ALL>(g, pv, fat, lng, src0, stride, use, p, i, acc);
+    else dslash_site_mrhs_t<M, SP, T, RP, ALL>(g, pv, fat, lng, src0, stride, use, p, i, acc);
+}
+
 template <int M, int SP, typename T, int RP>
 __device__ __forceinline__ void grouped_site(const Geom &g, int pv, const LinkSet &fat, const LinkSet &lng,
                                              const char *src0, size_t stride, unsigned use, int p, int i,
                                              T acc[RP][6])
 {
-    if constexpr (M != 0 && RP % 2 == 0) dslash_site_mrhs_pair<M, SP, RP>(g, pv, fat, lng, src0, stride, use, p, i, acc);
-    else dslash_site_mrhs_t<M, SP, T, RP>(g, pv, fat, lng, src0, stride, use, p, i, acc);
+    if (RP == 1 || use == (1u << RP) - 1u) grouped_site_of<M, SP, T, RP, true>(g, pv, fat, lng, src0, stride, use, p, i, acc);
+    else grouped_site_of<M, SP, T, RP, RP == 1>(g, pv, fat, lng, src0, stride, use, p, i, acc);
 }
 
 // Members per pass over a tile: every pass loads the links once for its members.  FP64 accumulators take twice the
-// registers, so FP64 passes take at most P64 members (1, 2 or 4, a tuned value): with 4 the FP64 kernel needs ~190
-// registers and one 256-thread CTA per SM, with 1 it keeps the single-system kernel's occupancy and reuses nothing.
-template <int M, int R, int P64> struct Pass { static constexpr int v = M == 0 ? (R < P64 ? R : P64) : R; };
+// registers, so FP64 passes take at most 4 members (1, 2 or 4, a tuned value): with 4 the FP64 kernel keeps 384 threads
+// per SM, with 1 it keeps the single-system kernel's occupancy and reuses nothing.
 
 // ---------------------------------------------------------------------------------------------------- kernels
 template <int BS>
@@ -254,7 +265,6 @@ __global__ void __launch_bounds__(BS) bk_init_kernel(const int2 *__restrict__ it
                 const bool finite = isfinite(tot);
                 st->status = finite ? 0 : KQ_STATUS_BREAKDOWN;
                 st->active[0] = (finite && tot > 0.0) ? 1 : 0;
-                if (!st->active[0] && st->running) atomicSub(st->running, 1);
                 st->ticket[0] = 0;
             }
         }
@@ -262,146 +272,173 @@ __global__ void __launch_bounds__(BS) bk_init_kernel(const int2 *__restrict__ it
     }
 }
 
-// Launch bounds of the dslash kernels: one group member (R = 1) keeps the single-system shapes (FP32: three
-// 256-thread CTAs per SM; FP64 and HALF up to 128 registers, at the 85-register cap the long-link row rebuild and
-// the HALF decode spill); several members need room for their accumulators (FP64: one 256-thread CTA per SM).  The
-// FP32 / HALF kernels of 2 or 4 members (dslash_site_mrhs_pair) are latency-bound and take three
-// 256-thread CTAs per SM at 80 registers (at most 32 B spilled); 8 members keep two (they would spill ~1 KB).
+// Launch bounds of the dslash kernels, in threads per SM: one group member (RP = 1) keeps the single-system shapes (FP32:
+// 768; FP64 and HALF 512, at the 85-register cap the long-link row rebuild and the HALF decode spill); several members
+// need registers for their accumulators and for the spinors in flight.  With the FP32 / HALF kernels of 2 and 4 members
+// held to 80 registers their second steps spilled 200 to 900 B: eight sources at 16^4, four per CTA, FP32 steps 35 and
+// 47 us at 768 threads per SM, 29 and 32 us at 512.
 template <int BS, int M, int RP> struct Bounds {
-    static constexpr int v = RP == 1 ? (M == 1 ? 768 : 512) / BS : (M == 0 ? 256 : RP <= 4 ? 768 : 512) / BS;
+    static constexpr int threads = RP == 1 ? (M == 1 ? 768 : 512) : M == 0 ? (RP == 2 ? 512 : 384) : RP == 2 ? 640 : RP == 4 ? 512 : 256;
+    static constexpr int v = threads / BS;
 };
+
+// Per-member scalar steps at the end of a tile: the partial sums v[r] of members G.mem[base + r], r in u, go to their
+// tile's slots, and the CTA that completes a member's last tile runs `step` on its total.  The members' sums and tickets
+// are taken side by side, by one thread each: one after another (a block sum, a fence and a ticket per member) they cost
+// about 2 us per member and tile.  Every thread of the CTA calls this.
+template <int BS, int RP, typename Step>
+__device__ __forceinline__ void member_steps(const GroupDesc &G, int base, unsigned u, int tile, int ticket,
+                                             const double (&v)[RP], double *sm, Step step)
+{
+    __shared__ double wsum[RP][BS / 32];
+    __shared__ unsigned done;
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+        double x = v[r];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if ((threadIdx.x & 31) == 0) wsum[r][threadIdx.x >> 5] = x;
+    }
+    if (threadIdx.x == 0) done = 0;
+    __syncthreads();
+    if (threadIdx.x < RP && (u >> threadIdx.x & 1u)) {
+        const SysDesc &d = c_sys[G.mem[base + threadIdx.x]];
+        double x = 0.0;
+#pragma unroll
+        for (int q = 0; q < BS / 32; ++q) x += wsum[threadIdx.x][q];
+        d.partials[tile] = x;
+        __threadfence();
+        if (atomicAdd(&d.st->ticket[ticket], 1u) == (unsigned)(d.ntiles - 1)) atomicOr(&done, 1u << threadIdx.x);
+    }
+    __syncthreads();
+    const unsigned fin = done;
+    if (fin) {
+        __threadfence();
+        for (int r = 0; r < RP; ++r)
+            if (fin >> r & 1u) {
+                const SysDesc &d = c_sys[G.mem[base + r]];
+                const double tot = tile_partials_sum(d.partials, d.ntiles, sm);
+                if (threadIdx.x == 0) {
+                    step(d.st, tot);
+                    d.st->ticket[ticket] = 0;
+                }
+            }
+    }
+    __syncthreads();  // wsum and done are free again
+}
 
 // K1: tmp_r = D p0_r and |tmp_r|^2 -> beta step with <p0, A p0> = sigma0 |p0|^2 + |tmp|^2 (|p0|^2 from the alpha
 // step's recurrence), for the members of each group whose operator precision is M (one launch per precision, so
-// that each launch is specialised; members in the other precisions are skipped).  In the FP32 / HALF phases p0 is
-// read from its copy in precision M.
-template <int BS, int M, int R, int P64>
-__global__ void __launch_bounds__(BS, Bounds<BS, M, Pass<M, R, P64>::v>::v) bk_dslash1_kernel(
-    const int2 *__restrict__ items, int nitems, int spt)
+// that each launch is specialised; members in the other precisions are skipped), RP members per pass over the tile.  In
+// the FP32 / HALF phases p0 is read from its copy in precision M.
+template <int BS, int M, int RP>
+__global__ void __launch_bounds__(BS, Bounds<BS, M, RP>::v) bk_dslash1_kernel(const int2 *__restrict__ items, int nitems,
+                                                                              int spt)
 {
     typedef typename Acc2<M, M>::T T;
-    constexpr int RP = Pass<M, R, P64>::v;
     __shared__ double sm[32];
 #pragma unroll 1
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const int2 w = items[it];
         const GroupDesc &G = c_grp[w.x];
-        const unsigned use = group_mask<R, M>(G);
+        const unsigned use = group_mask<M>(G);
         if (!use) continue;
         const SysDesc &d0 = c_sys[G.mem[0]];
-        double tt[R];
+        // the FP32 / HALF phases gather p0 from its copy in their own precision (a third or half of the FP64 bytes
+        // through L1/L2 for each of the members)
+        const char *src = static_cast<const char *>(M == 0 ? d0.p0 : d0.p0s);
+        const size_t vbx = M == 0 ? d0.vb : d0.vbs;
+#pragma unroll 1
+        for (int base = 0; base < G.n; base += RP) {
+            const unsigned u = (use >> base) & ((1u << RP) - 1u);
+            if (!u) continue;
+            double tt[RP];
 #pragma unroll
-        for (int r = 0; r < R; ++r) tt[r] = 0.0;
-        for (int sidx = 0; sidx < spt; ++sidx) {
-            const int i = tile_site<BS>(w.y, spt, sidx);
-            if (i >= d0.g.vh) break;
-#pragma unroll
-            for (int base = 0; base < R; base += RP) {
-                const unsigned u = (use >> base) & ((1u << RP) - 1u);
-                if (!u) continue;
+            for (int r = 0; r < RP; ++r) tt[r] = 0.0;
+#pragma unroll 1
+            for (int sidx = 0; sidx < spt; ++sidx) {
+                const int i = tile_site<BS>(w.y, spt, sidx);
+                if (i >= d0.g.vh) break;
                 T acc[RP][6];
-                // the FP32 / HALF phases gather p0 from its copy in their own precision (a third or half of the
-                // FP64 bytes through L1/L2 for each of the RP members)
-                const char *src = static_cast<const char *>(M == 0 ? d0.p0 : d0.p0s);
-                const size_t vbx = M == 0 ? d0.vb : d0.vbs;
-                grouped_site<M, M, T, RP>(d0.g, d0.pv, d0.fat[M], d0.lng[M], src + base * vbx, vbx, u,
-                                                1 - d0.parity, i, acc);
+                grouped_site<M, M, T, RP>(d0.g, d0.pv, d0.fat[M], d0.lng[M], src + base * vbx, vbx, u, 1 - d0.parity, i,
+                                          acc);
 #pragma unroll
                 for (int r = 0; r < RP; ++r)
                     if (u & (1u << r)) {
                         st_spinor_as<M>(static_cast<char *>(d0.tmp) + (base + r) * d0.vb, d0.pv, i, acc[r]);
 #pragma unroll
-                        for (int k = 0; k < 6; ++k) tt[base + r] += (double)acc[r][k] * (double)acc[r][k];
+                        for (int k = 0; k < 6; ++k) tt[r] += (double)acc[r][k] * (double)acc[r][k];
                     }
             }
+            member_steps<BS, RP>(G, base, u, w.y, 1, tt, sm, [](MsState *st, double tot) {
+                ms_beta(st, 0, st->rNorm2, st->shift[0] * st->pp + tot);
+            });
         }
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-            if (use & (1u << r)) {
-                const SysDesc &d = c_sys[G.mem[r]];
-                MsState *st = d.st;
-                const double bt = block_sum(tt[r], sm);
-                if (threadIdx.x == 0) d.partials[w.y] = bt;
-                if (tile_ticket_last(&st->ticket[1], d.ntiles)) {
-                    const double tot = tile_partials_sum(d.partials, d.ntiles, sm);
-                    if (threadIdx.x == 0) {
-                        ms_beta(st, 0, st->rNorm2, st->shift[0] * st->pp + tot);
-                        st->ticket[1] = 0;
-                    }
-                }
-                __syncthreads();
-            }
     }
 }
 
 // K2: r_r^(i+1) = r_r^(i) + B0 (sigma0 p0_r - D tmp_r) into each member's ring (s stays in registers), |r_r|^2 ->
-// alpha step, for the members in precision M.  The alpha step picks the next iteration's precision in next_mode,
-// applied in K3, so the K2 launches of the other precisions in this iteration do not pick the system up again.
-template <int BS, int M, int R, int P64>
-__global__ void __launch_bounds__(BS, Bounds<BS, M, Pass<M, R, P64>::v>::v) bk_dslash2_kernel(
-    const int2 *__restrict__ items, int nitems, int spt)
+// alpha step, for the members in precision M.  The alpha step picks the next precision in next_mode, applied in K3 at
+// the end of a chunk.
+template <int BS, int M, int RP>
+__global__ void __launch_bounds__(BS, Bounds<BS, M, RP>::v) bk_dslash2_kernel(const int2 *__restrict__ items, int nitems,
+                                                                              int spt)
 {
     typedef typename Acc2<M, M>::T T;
-    constexpr int RP = Pass<M, R, P64>::v;
     __shared__ double sm[32];
 #pragma unroll 1
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const int2 w = items[it];
         const GroupDesc &G = c_grp[w.x];
-        const unsigned use = group_mask<R, M>(G);
+        const unsigned use = group_mask<M>(G);
         if (!use) continue;
         const SysDesc &d0 = c_sys[G.mem[0]];
-        double nn[R];
+#pragma unroll 1
+        for (int base = 0; base < G.n; base += RP) {
+            const unsigned u = (use >> base) & ((1u << RP) - 1u);
+            if (!u) continue;
+            double nn[RP];
 #pragma unroll
-        for (int r = 0; r < R; ++r) nn[r] = 0.0;
-        for (int sidx = 0; sidx < spt; ++sidx) {
-            const int i = tile_site<BS>(w.y, spt, sidx);
-            if (i >= d0.g.vh) break;
-#pragma unroll
-            for (int base = 0; base < R; base += RP) {
-                const unsigned u = (use >> base) & ((1u << RP) - 1u);
-                if (!u) continue;
+            for (int r = 0; r < RP; ++r) nn[r] = 0.0;
+#pragma unroll 1
+            for (int sidx = 0; sidx < spt; ++sidx) {
+                const int i = tile_site<BS>(w.y, spt, sidx);
+                if (i >= d0.g.vh) break;
                 T acc[RP][6];
                 grouped_site<M, M, T, RP>(d0.g, d0.pv, d0.fat[M], d0.lng[M],
-                                                static_cast<const char *>(d0.tmp) + base * d0.vb, d0.vb, u,
-                                                d0.parity, i, acc);
+                                          static_cast<const char *>(d0.tmp) + base * d0.vb, d0.vb, u, d0.parity, i, acc);
+                // two members' p0 and r are loaded before either's new r is stored
+                constexpr int NB = RP < 2 || M > 0 ? 1 : 2;
 #pragma unroll
-                for (int r = 0; r < RP; ++r)
-                    if (u & (1u << r)) {
-                        const SysDesc &d = c_sys[G.mem[base + r]];
-                        const MsState *st = d.st;
-                        const int itc = st->iter;
-                        const char *rin = static_cast<const char *>(d.ring) + (size_t)(itc % kWin) * d.vb;
-                        char *rout = static_cast<char *>(d.ring) + (size_t)((itc + 1) % kWin) * d.vb;
-                        double pv6[6], rv[6];
-                        ld_spinor<0>(d.p0, d.pv, i, pv6);
-                        ld_spinor<0>(rin, d.pv, i, rv);
-                        const double sig = st->shift[0], b0 = st->b0;
+                for (int r0 = 0; r0 < RP; r0 += NB) {
+                    double pv6[NB][6], rv[NB][6];
 #pragma unroll
-                        for (int k = 0; k < 6; ++k) {
-                            rv[k] += b0 * (sig * pv6[k] - (double)acc[r][k]);
-                            nn[base + r] += rv[k] * rv[k];
+                    for (int q = 0; q < NB; ++q)
+                        if (u & (1u << (r0 + q))) {
+                            const SysDesc &d = c_sys[G.mem[base + r0 + q]];
+                            ld_spinor<0>(d.p0, d.pv, i, pv6[q]);
+                            ld_spinor<0>(static_cast<const char *>(d.ring) + (size_t)(d.st->iter % kWin) * d.vb, d.pv, i,
+                                         rv[q]);
                         }
-                        st_spinor<0>(rout, d.pv, i, rv);
-                    }
-            }
-        }
 #pragma unroll
-        for (int r = 0; r < R; ++r)
-            if (use & (1u << r)) {
-                const SysDesc &d = c_sys[G.mem[r]];
-                MsState *st = d.st;
-                const double bn = block_sum(nn[r], sm);
-                if (threadIdx.x == 0) d.partials[w.y] = bn;
-                if (tile_ticket_last(&st->ticket[2], d.ntiles)) {
-                    const double tot = tile_partials_sum(d.partials, d.ntiles, sm);
-                    if (threadIdx.x == 0) {
-                        ms_alpha(st, st->rNorm2, tot);
-                        st->ticket[2] = 0;
-                    }
+                    for (int q = 0; q < NB; ++q)
+                        if (u & (1u << (r0 + q))) {
+                            const SysDesc &d = c_sys[G.mem[base + r0 + q]];
+                            const MsState *st = d.st;
+                            const double sig = st->shift[0], b0 = st->b0;
+#pragma unroll
+                            for (int k = 0; k < 6; ++k) {
+                                rv[q][k] += b0 * (sig * pv6[q][k] - (double)acc[r0 + q][k]);
+                                nn[r0 + q] += rv[q][k] * rv[q][k];
+                            }
+                            st_spinor<0>(static_cast<char *>(d.ring) + (size_t)((st->iter + 1) % kWin) * d.vb, d.pv, i,
+                                         rv[q]);
+                        }
                 }
-                __syncthreads();
             }
+            member_steps<BS, RP>(G, base, u, w.y, 2, nn, sm,
+                                 [](MsState *st, double tot) { ms_alpha(st, st->rNorm2, tot); });
+        }
     }
 }
 
@@ -628,7 +665,7 @@ __global__ void __launch_bounds__(BS, Bounds<BS, M, 1>::v) bk_dslash1_staged_ker
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const int2 w = items[it];
         const GroupDesc &G = c_grp[w.x];
-        const unsigned use = group_mask<R, M>(G);
+        const unsigned use = group_mask<M>(G);
         if (!use) continue;
         const SysDesc &d0 = c_sys[G.mem[0]];
         const char *src = static_cast<const char *>(d0.p0) + r * d0.vb;
@@ -664,7 +701,7 @@ __global__ void __launch_bounds__(BS, Bounds<BS, M, 1>::v) bk_dslash2_staged_ker
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const int2 w = items[it];
         const GroupDesc &G = c_grp[w.x];
-        const unsigned use = group_mask<R, M>(G);
+        const unsigned use = group_mask<M>(G);
         if (!use) continue;
         const SysDesc &d0 = c_sys[G.mem[0]];
         const bool mine = (use >> r) & 1u;
@@ -697,9 +734,10 @@ __global__ void __launch_bounds__(BS, Bounds<BS, M, 1>::v) bk_dslash2_staged_ker
 }
 
 // K3: p0 = r^(i) + a0 p0 (and its copy in the next iteration's precision when that is FP32 or HALF); the system's
-// last tile takes the shift step, and the next iteration's precision takes effect.
+// last tile takes the shift step.  Precisions change with the last iteration of a chunk only, so that the host knows
+// which dslash launches the next chunk needs.
 template <int BS>
-__global__ void __launch_bounds__(BS) bk_p0_kernel(const int2 *__restrict__ items, int nitems, int spt)
+__global__ void __launch_bounds__(BS) bk_p0_kernel(const int2 *__restrict__ items, int nitems, int spt, int last)
 {
 #pragma unroll 1
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
@@ -709,7 +747,7 @@ __global__ void __launch_bounds__(BS) bk_p0_kernel(const int2 *__restrict__ item
         if (!st->active[0]) continue;
         const char *r = static_cast<const char *>(d.ring) + (size_t)(st->iter % kWin) * d.vb;
         const double a0 = st->a0;
-        const int nm = st->next_mode;  // the next iteration's operator precision (set by the alpha step)
+        const int nm = last ? st->next_mode : st->mode;  // the next iteration's operator precision
         for (int sidx = 0; sidx < spt; ++sidx) {
             const int i = tile_site<BS>(w.y, spt, sidx);
             if (i >= d.g.vh) break;
@@ -726,15 +764,33 @@ __global__ void __launch_bounds__(BS) bk_p0_kernel(const int2 *__restrict__ item
         if (tile_ticket_last(&st->ticket[3], d.ntiles)) {
             const bool go = ms_shift_step(st);
             if (threadIdx.x == 0) {
-                if (!go) {
-                    st->active[0] = 0;
-                    if (st->running) atomicSub(st->running, 1);
-                }
-                st->mode = st->next_mode;
+                if (!go) st->active[0] = 0;
+                st->mode = nm;
                 st->ticket[3] = 0;
             }
         }
         __syncthreads();
+    }
+}
+
+// End of a chunk: the number of systems still iterating and the precisions they will iterate in (bit m: precision m),
+// written to the host's page.  One block.
+__global__ void __launch_bounds__(kMaxBatch) bk_poll_kernel(int nsys, volatile int *host)
+{
+    __shared__ int running, modes;
+    if (threadIdx.x == 0) running = modes = 0;
+    __syncthreads();
+    if ((int)threadIdx.x < nsys) {
+        const MsState *st = c_sys[threadIdx.x].st;
+        if (st->active[0]) {
+            atomicAdd(&running, 1);
+            atomicOr(&modes, 1 << st->mode);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        host[0] = running;
+        host[1] = modes;
     }
 }
 
@@ -784,6 +840,8 @@ struct BatchItems {
     int nsys;
     const int2 *grp;
     int ngrp;
+    int systems;
+    int *host;  // page-locked, written at the end of every chunk: systems still iterating, their precisions
 };
 
 template <int BS>
@@ -819,48 +877,70 @@ static cudaError_t staged_attrs()
     return cudaSuccess;
 }
 
-template <int BS, int R, int P64>
-static void enqueue_batch_chunk_r(const BatchItems &it, int grid, int spt, cudaStream_t s)
+// modes: the precisions some system iterates in during the chunk (a launch no system takes part in costs 2.2 us; with
+// all three in every step they were 3.3 of the 54 ms of eight 16^4 systems)
+template <int BS, int M, int RP>
+static void enqueue_dslash(int step, const BatchItems &it, int grid, int spt, cudaStream_t s)
 {
-    for (int k = 0; k < kChunk; ++k) {
-        // (P64 only shapes the FP64 kernels, 0 = staged; the sloppy ones are instantiated once)
-        if constexpr (P64 == 0)
-            bk_dslash1_staged_kernel<BS, 0, R><<<grid, BS, staged_smem<0>(BS / R), s>>>(it.grp, it.ngrp, spt);
-        else bk_dslash1_kernel<BS, 0, R, P64><<<grid, BS, 0, s>>>(it.grp, it.ngrp, spt);
-        bk_dslash1_kernel<BS, 1, R, 1><<<grid, BS, 0, s>>>(it.grp, it.ngrp, spt);
-        bk_dslash1_kernel<BS, 2, R, 1><<<grid, BS, 0, s>>>(it.grp, it.ngrp, spt);
-        if constexpr (P64 == 0)
-            bk_dslash2_staged_kernel<BS, 0, R><<<grid, BS, staged_smem<0>(BS / R), s>>>(it.grp, it.ngrp, spt);
-        else bk_dslash2_kernel<BS, 0, R, P64><<<grid, BS, 0, s>>>(it.grp, it.ngrp, spt);
-        bk_dslash2_kernel<BS, 1, R, 1><<<grid, BS, 0, s>>>(it.grp, it.ngrp, spt);
-        bk_dslash2_kernel<BS, 2, R, 1><<<grid, BS, 0, s>>>(it.grp, it.ngrp, spt);
-        bk_p0_kernel<BS><<<grid, BS, 0, s>>>(it.sys, it.nsys, spt);
-    }
-    bk_window_kernel<BS><<<grid, BS, 0, s>>>(it.sys, it.nsys, spt);
+    if (step == 1) bk_dslash1_kernel<BS, M, RP><<<grid, BS, 0, s>>>(it.grp, it.ngrp, spt);
+    else bk_dslash2_kernel<BS, M, RP><<<grid, BS, 0, s>>>(it.grp, it.ngrp, spt);
 }
 
 template <int BS, int R>
-static void enqueue_batch_chunk_p(const BatchItems &it, int grid, int spt, int p64, cudaStream_t s)
+static void enqueue_staged(int step, const BatchItems &it, int grid, int spt, cudaStream_t s)
 {
-    if constexpr (staged_ok(BS, R))
-        if (p64 == 0) {
-            enqueue_batch_chunk_r<BS, R, 0>(it, grid, spt, s);
-            return;
-        }
-    if (R == 1 || p64 == 1) enqueue_batch_chunk_r<BS, R, 1>(it, grid, spt, s);
-    else if (R == 2 || p64 == 2) enqueue_batch_chunk_r<BS, R, 2>(it, grid, spt, s);
-    else enqueue_batch_chunk_r<BS, R, 4>(it, grid, spt, s);
+    if constexpr (staged_ok(BS, R)) {
+        const size_t sm = staged_smem<0>(BS / R);
+        if (step == 1) bk_dslash1_staged_kernel<BS, 0, R><<<grid, BS, sm, s>>>(it.grp, it.ngrp, spt);
+        else bk_dslash2_staged_kernel<BS, 0, R><<<grid, BS, sm, s>>>(it.grp, it.ngrp, spt);
+    }
 }
 
+// dslash step 1 or 2 of the systems in precision m, for groups of at most rhs members (p64: members per pass in FP64)
 template <int BS>
-static void enqueue_batch_chunk(const BatchItems &it, int grid, int rhs, int spt, int p64, cudaStream_t s)
+static void enqueue_batch_step(int step, int m, const BatchItems &it, int grid, int rhs, int spt, int p64, cudaStream_t s)
 {
-    switch (rhs) {
-        case 8: enqueue_batch_chunk_p<BS, 8>(it, grid, spt, p64, s); break;
-        case 4: enqueue_batch_chunk_p<BS, 4>(it, grid, spt, p64, s); break;
-        case 2: enqueue_batch_chunk_p<BS, 2>(it, grid, spt, p64, s); break;
-        default: enqueue_batch_chunk_r<BS, 1, 1>(it, grid, spt, s); break;
+    if (m == 0 && p64 == 0 && staged_ok(BS, rhs)) {
+        switch (rhs) {
+            case 8: enqueue_staged<BS, 8>(step, it, grid, spt, s); break;
+            case 4: enqueue_staged<BS, 4>(step, it, grid, spt, s); break;
+            default: enqueue_staged<BS, 2>(step, it, grid, spt, s); break;
+        }
+        return;
     }
+    const int rp = m == 0 ? std::min(rhs, p64 == 0 ? 4 : p64) : rhs;
+#define KQ_STEP(Mv, RPv) enqueue_dslash<BS, Mv, RPv>(step, it, grid, spt, s)
+    if (m == 0) {
+        if (rp >= 4) KQ_STEP(0, 4);
+        else if (rp == 2) KQ_STEP(0, 2);
+        else KQ_STEP(0, 1);
+    } else if (m == 1) {
+        if (rp >= 8) KQ_STEP(1, 8);
+        else if (rp == 4) KQ_STEP(1, 4);
+        else if (rp == 2) KQ_STEP(1, 2);
+        else KQ_STEP(1, 1);
+    } else {
+        if (rp >= 8) KQ_STEP(2, 8);
+        else if (rp == 4) KQ_STEP(2, 4);
+        else if (rp == 2) KQ_STEP(2, 2);
+        else KQ_STEP(2, 1);
+    }
+#undef KQ_STEP
+}
+
+// modes: the precisions some system iterates in during the chunk (a launch no system takes part in costs 2.2 us; with
+// all three in every step they were 3.3 of the 54 ms of eight 16^4 systems)
+template <int BS>
+static void enqueue_batch_chunk(const BatchItems &it, int grid, int rhs, int spt, int p64, int modes, cudaStream_t s)
+{
+    for (int k = 0; k < kChunk; ++k) {
+        for (int step = 1; step <= 2; ++step)
+            for (int m = 0; m < 3; ++m)
+                if (modes & (1 << m)) enqueue_batch_step<BS>(step, m, it, grid, rhs, spt, p64, s);
+        bk_p0_kernel<BS><<<grid, BS, 0, s>>>(it.sys, it.nsys, spt, k == kChunk - 1 ? 1 : 0);
+    }
+    bk_window_kernel<BS><<<grid, BS, 0, s>>>(it.sys, it.nsys, spt);
+    bk_poll_kernel<<<1, kMaxBatch, 0, s>>>(it.systems, it.host);
 }
 
 }  // namespace kq
@@ -882,8 +962,7 @@ struct kq_batch {
     std::vector<BatchSystem> sys;
     void *work = nullptr;
     size_t work_bytes = 0;
-    int *d_running = nullptr;
-    int *h_running = nullptr;  // pinned
+    int *h_running = nullptr;  // pinned: systems still iterating, the precisions they iterate in
     int2 *d_items = nullptr;   // per-system items, then per-group items
     size_t items_cap = 0;
 };
@@ -898,7 +977,6 @@ KQ_API KuQCDStatus kq_batch_create(int device, kq_batch **out)
     b->device = device;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_running, sizeof(int) * 4);
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_running, sizeof(int) * 4);
     if (e != cudaSuccess) {
         set_last_error(std::string("kq_batch_create: ") + cudaGetErrorString(e));
@@ -916,7 +994,6 @@ KQ_API void kq_batch_destroy(kq_batch *b)
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->work) cudaFree(b->work);
     if (b->d_items) cudaFree(b->d_items);
-    if (b->d_running) cudaFree(b->d_running);
     if (b->h_running) cudaFreeHost(b->h_running);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
@@ -1084,7 +1161,6 @@ cudaError_t batch_plan(kq_batch *b, int bs, int rhs, int spt, BatchPlan &plan, b
             } else {
                 h.tol = S.param.tol;
             }
-            h.running = b->d_running;
         }
     }
     for (size_t si = 0; si < b->sys.size(); ++si)
@@ -1111,7 +1187,7 @@ static KuQCDStatus solve_batched(kq_batch *b, kq_batch_info *out)
     }
 
     // launch shape: tuned once per batch signature (sizes, shared gauge fields, shifts, schedule), cached on disk
-    std::string key = "batch7";
+    std::string key = "batch8";
     for (auto &S : b->sys) {
         int owner = 0;  // first system on the same context: systems sharing links share this number
         while (b->sys[owner].ctx != S.ctx) ++owner;
@@ -1172,9 +1248,7 @@ static KuQCDStatus solve_batched(kq_batch *b, kq_batch_info *out)
                                     cudaMemcpyHostToDevice, s));
         for (size_t i = 0; i < nsys; ++i)
             KQ_CUDA_TRY(cudaMemcpyAsync(plan.desc[i].st, &plan.init[i], sizeof(MsState), cudaMemcpyHostToDevice, s));
-        const int nsys_i = (int)nsys;
-        KQ_CUDA_TRY(cudaMemcpyAsync(b->d_running, &nsys_i, sizeof(int), cudaMemcpyHostToDevice, s));
-        const BatchItems items{b->d_items, (int)nsi, b->d_items + nsi, (int)ngi};
+        const BatchItems items{b->d_items, (int)nsi, b->d_items + nsi, (int)ngi, (int)nsys, b->h_running};
         const int grid = std::max(1, std::min((int)nsi, dev_sms * t.ctas_per_sm));
         *ngroups = (int)plan.groups.size();
         cudaEvent_t e0, e1;
@@ -1183,38 +1257,55 @@ static KuQCDStatus solve_batched(kq_batch *b, kq_batch_info *out)
         if (t.bs == 128) enqueue_batch_init<128>(items, grid, t.spt, s);
         else enqueue_batch_init<256>(items, grid, t.spt, s);
         KQ_CUDA_TRY(cudaGetLastError());
-        *launches = 1;
-        cudaGraph_t graph = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        KQ_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        if (t.bs == 128) enqueue_batch_chunk<128>(items, grid, t.rhs, t.spt, t.p64, s);
-        else enqueue_batch_chunk<256>(items, grid, t.rhs, t.spt, t.p64, s);
-        cudaError_t ee = cudaStreamEndCapture(s, &graph);
-        if (ee == cudaSuccess) ee = cudaGraphInstantiate(&exec, graph, 0);
-        if (graph) cudaGraphDestroy(graph);
-        KQ_CUDA_TRY(ee);
+        bk_poll_kernel<<<1, kMaxBatch, 0, s>>>((int)nsys, b->h_running);
+        *launches = 2;
+        auto enqueue = [&](int modes) {
+            if (t.bs == 128) enqueue_batch_chunk<128>(items, grid, t.rhs, t.spt, t.p64, modes, s);
+            else enqueue_batch_chunk<256>(items, grid, t.rhs, t.spt, t.p64, modes, s);
+        };
+        // one graph per set of precisions; the first chunk of a set is enqueued kernel by kernel and its graph built
+        // while it runs
+        cudaGraphExec_t exec[8] = {nullptr};
+        auto build = [&](int modes) -> cudaError_t {
+            cudaGraph_t graph = nullptr;
+            KQ_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+            enqueue(modes);
+            cudaError_t ee = cudaStreamEndCapture(s, &graph);
+            if (ee == cudaSuccess) ee = cudaGraphInstantiate(&exec[modes], graph, 0);
+            if (graph) cudaGraphDestroy(graph);
+            return ee;
+        };
         int chunks = 0;
         int chunk_cap = 8;
         for (const MsState &h : plan.init) chunk_cap = std::max(chunk_cap, h.max_iter / kChunk + 8);
         cudaError_t err = cudaSuccess;
-        cudaEventRecord(e0, s);  // device time of the iterations (after the init kernel and graph set-up)
+        cudaEventRecord(e0, s);  // device time of the iterations (after the init kernel)
         for (;;) {
-            err = cudaMemcpyAsync(b->h_running, b->d_running, sizeof(int), cudaMemcpyDeviceToHost, s);
-            if (err == cudaSuccess) err = cudaStreamSynchronize(s);
-            if (err != cudaSuccess || *b->h_running <= 0) break;
+            err = cudaStreamSynchronize(s);
+            if (err != cudaSuccess || b->h_running[0] <= 0) break;
             if (max_chunks > 0 && chunks >= max_chunks) break;
-            err = cudaGraphLaunch(exec, s);
+            const int modes = b->h_running[1] & 7;
+            if (exec[modes]) {
+                err = cudaGraphLaunch(exec[modes], s);
+            } else {
+                enqueue(modes);
+                err = cudaGetLastError();
+                if (err == cudaSuccess) err = build(modes);
+            }
             if (err != cudaSuccess) break;
             ++chunks;
-            *launches += 7 * kChunk + 1;  // two dslash steps x three precisions + p0 per iteration, + window
+            // two dslash steps per precision + p0 per iteration, + window and poll
+            *launches += kChunk * (2 * ((modes & 1) + (modes >> 1 & 1) + (modes >> 2)) + 1) + 2;
             if (chunks > chunk_cap) break;  // every system has stopped by then while the states are consistent
         }
+        if (err != cudaSuccess) cudaStreamSynchronize(s);
         cudaEventRecord(e1, s);
         cudaEventSynchronize(e1);
         cudaEventElapsedTime(ms_out, e0, e1);
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        cudaGraphExecDestroy(exec);
+        for (auto &x : exec)
+            if (x) cudaGraphExecDestroy(x);
         *chunks_out = chunks;
         return err;
     };

@@ -27,7 +27,6 @@ struct MsState {
     double d[kMaxShift][kWin], f[kMaxShift][kWin];  // coefficients of the ring residuals
     int mode, next_mode;  // batched solver: operator precision of this / the next iteration (0 FP64, 1 FP32, 2 HALF)
     double rho32_2, rho16_2;  // squared relative-residual switch points (0: never)
-    int *running;             // batched solver: systems still iterating (decremented when this one stops)
 };
 
 struct MsPoll {  // the first words of MsState

@@ -31,14 +31,18 @@ std::string cache_path()
 
 std::string gpu_name()
 {
+    // asked once per device (under g_mu): the properties query takes about 2.5 ms
+    static std::map<int, std::string> names;
     int dev = 0;
     cudaGetDevice(&dev);
+    auto it = names.find(dev);
+    if (it != names.end()) return it->second;
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return "unknown";
     std::string n = prop.name;
     for (char &c : n)
         if (c == ' ' || c == '|') c = '_';
-    return n;
+    return names[dev] = n;
 }
 
 void load_locked()
