@@ -40,8 +40,10 @@ __global__ void __launch_bounds__(256, MB) dslash_xmy_kernel(Geom g, int pv, Lin
 }
 
 // Full-lattice (non-preconditioned, KUQCD_HISQ_DIRAC) operator: a full field is the parity-0 field followed by the
-// parity-1 field, `half` bytes apart.  blockIdx.y = output parity p; the input is the other half.  dst = D src on
-// both parities in one launch (dirac_hisq.cpp:128-136, 418-424 with offseti = offsetg = 0), or, with pvec,
+// parity-1 field, `half` bytes apart.  blockIdx.x & 1 = output parity p; the input is the other half.  Every link is used
+// twice, by the forward hop at its site and by the backward hop of a neighbour of the other parity: with the parities
+// interleaved the second use comes while the link is still in the L2 (one parity after the other: a field later).
+// dst = D src on both parities in one launch (dirac_hisq.cpp:128-136, 418-424 with offseti = offsetg = 0), or, with pvec,
 // dst = sigma * pvec - D src (the second half of sigma - D D).
 template <int LP, int SP, int MB>
 __global__ void __launch_bounds__(256, MB) dslash_full_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
@@ -49,11 +51,11 @@ __global__ void __launch_bounds__(256, MB) dslash_full_kernel(Geom g, int pv, Li
                                                           char *__restrict__ dst, size_t half, double sigma)
 {
     using T = typename Acc2<LP, SP>::T;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x >> 1) * blockDim.x + threadIdx.x;
     if (i >= g.vh) return;
-    const int p = blockIdx.y;
+    const int p = blockIdx.x & 1;
     T acc[6];
-    dslash_site2<LP, SP>(g, pv, fat, lng, src + (1 - p) * half, p, i, acc);
+    dslash_site2<LP, SP, true>(g, pv, fat, lng, src + (1 - p) * half, p, i, acc);
     if (pvec) {
         T pv6[6];
         ld_spinor<SP>(pvec + p * half, pv, i, pv6);
@@ -64,7 +66,7 @@ __global__ void __launch_bounds__(256, MB) dslash_full_kernel(Geom g, int pv, Li
 }
 
 // The three forms above with S threads per site (dslash_site_split): dst = D src on parity p, or on both parities
-// (half > 0: full-lattice fields, blockIdx.y = p), or sigma * pvec - D src when pvec is given.
+// (half > 0: full-lattice fields, blockIdx.x & 1 = p), or sigma * pvec - D src when pvec is given.
 template <int LP, int SP, int S>
 __global__ void __launch_bounds__(S *split_sites(S)) dslash_split_kernel(Geom g, int pv, LinkSet fat, LinkSet lng,
                                                                          const char *src, const char *pvec, char *dst,
@@ -75,8 +77,8 @@ __global__ void __launch_bounds__(S *split_sites(S)) dslash_split_kernel(Geom g,
     using T = typename Acc2<LP, SP>::T;
     constexpr int NS = split_sites(S);
     __shared__ T part[(S - 1) * 6 * NS];
-    const int i = blockIdx.x * NS + threadIdx.x % NS;
-    const int par = half ? (int)blockIdx.y : p;
+    const int i = (half ? blockIdx.x >> 1 : blockIdx.x) * NS + threadIdx.x % NS;
+    const int par = half ? (int)(blockIdx.x & 1) : p;
     T acc[6];
     bool on;
     const auto ready = [&] {
@@ -141,7 +143,7 @@ static cudaError_t launch_split(int S, const Geom &g, const GaugeDev &gd, const 
                                 size_t half, int p, double sigma, const int *gate, cudaStream_t s, bool follows = false)
 {
     const int ns = split_sites(S);
-    const dim3 grid((g.vh + ns - 1) / ns, half ? 2 : 1);
+    const dim3 grid((g.vh + ns - 1) / ns * (half ? 2 : 1));
     const int pv = pad_sites(g.vh), bs = S * ns;
     auto a = static_cast<const char *>(src);
     auto b = static_cast<const char *>(pvec);
@@ -238,7 +240,7 @@ cudaError_t launch_dslash_full(const Geom &g, const GaugeDev &gd, int prec, cons
         KQ_DISPATCH_PAIR(prec, prec, e = (launch_split<LP, SP>(S, g, gd, src, pvec, dst, half, 0, sigma, nullptr, s, pvec != nullptr)));
         return e;
     }
-    const dim3 grid((g.vh + 255) / 256, 2);
+    const dim3 grid((g.vh + 255) / 256 * 2);
     const int pv = pad_sites(g.vh);
     auto S = static_cast<const char *>(src);
     auto Pv = static_cast<const char *>(pvec);

@@ -88,17 +88,17 @@ __device__ __forceinline__ int nbr_index(const Geom &g, const SiteCoord &c, int 
 // One link as type T.  HALF links (LP = 2) come back as raw int16 values: a site's fat-link terms are accumulated
 // in units of the fat field's scale, the long-link terms have their spinor multiplied by scale_long / scale_fat
 // (6 products instead of 18 on the link), and the sum is scaled once at the end (fold_scale_*).
-template <int LP, typename T>
+template <int LP, typename T, bool KEEP = false>
 __device__ __forceinline__ void ld_link_fold(const void *base, int pv, int dir, int i, const LinkSet &L, T u[18])
 {
     if constexpr (LP == 2) {
         float q[18];
-        ld_link_q16(base, pv, dir, i, q);
+        ld_link_q16<KEEP>(base, pv, dir, i, q);
 #pragma unroll
         for (int k = 0; k < 18; ++k) u[k] = (T)q[k];
     } else {
         typename Acc<LP>::T w[18];
-        ld_link_any<LP>(base, pv, dir, i, L.scale, L.recon, w);
+        ld_link_any<LP, KEEP>(base, pv, dir, i, L.scale, L.recon, w);
 #pragma unroll
         for (int k = 0; k < 18; ++k) u[k] = (T)w[k];
     }
@@ -133,8 +133,9 @@ __device__ __forceinline__ void fold_long_spinor(T rl, T v[6])
 template <int LP, int SP> struct Acc2 { using T = float; };
 template <> struct Acc2<0, 0> { using T = double; };
 
-// acc = (D src)(i) for output parity p.  src is the parity-(1-p) field.  Links in precision LP, spinors in SP.
-template <int LP, int SP>
+// acc = (D src)(i) for output parity p.  src is the parity-(1-p) field.  Links in precision LP, spinors in SP.  KEEP: the
+// forward links will be read again, by the backward hops of the other parity's sites in the same launch.
+template <int LP, int SP, bool KEEP = false>
 __device__ __forceinline__ void dslash_site2(const Geom &g, int pv, const LinkSet &fat, const LinkSet &lng,
                                              const void *src, int p, int i, typename Acc2<LP, SP>::T acc[6])
 {
@@ -155,10 +156,10 @@ __device__ __forceinline__ void dslash_site2(const Geom &g, int pv, const LinkSe
         const int nb1 = nbr_index(g, c, i, dir, -1);
         const int nb3 = nbr_index(g, c, i, dir, -3);
         T u[18], v[6];
-        ld_link_fold<LP>(fat_p, pv, dir, i, fat, u);
+        ld_link_fold<LP, T, KEEP>(fat_p, pv, dir, i, fat, u);
         ld_spinor<SP>(src, pv, nf1, v);
         mv_add(u, v, acc);
-        ld_link_fold<LP>(lng_p, pv, dir, i, lng, u);
+        ld_link_fold<LP, T, KEEP>(lng_p, pv, dir, i, lng, u);
         ld_spinor<SP>(src, pv, nf3, v);
         fold_long_spinor<LP>(rl, v);
         mv_add(u, v, acc);

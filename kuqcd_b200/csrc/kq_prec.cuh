@@ -11,12 +11,14 @@ constexpr int kPad = 64;
 __host__ __device__ inline int pad_sites(int vh) { return (vh + kPad - 1) / kPad * kPad; }
 
 // ------------------------------------------------------------------------------------------------ load helpers
-// Links are read once per dslash: stream them (evict-first) so the L2 keeps the re-read spinor neighbours.
-__device__ __forceinline__ double2 ld_stream(const double2 *p) { return __ldcs(p); }
-__device__ __forceinline__ float4 ld_stream(const float4 *p) { return __ldcs(p); }
-__device__ __forceinline__ float2 ld_stream(const float2 *p) { return __ldcs(p); }
-__device__ __forceinline__ int4 ld_stream(const int4 *p) { return __ldcs(p); }
-__device__ __forceinline__ int ld_stream(const int *p) { return __ldcs(p); }
+// Links are read once per even-odd dslash: stream them (evict-first) so the L2 keeps the re-read spinor neighbours.  The
+// full-lattice dslash reads every link twice; its first reads keep the line (KEEP).
+template <bool KEEP = false, typename V>
+__device__ __forceinline__ V ld_stream(const V *p)
+{
+    if constexpr (KEEP) return __ldg(p);
+    else return __ldcs(p);
+}
 
 // int16 fixed point: q = rint(v * 32767 / scale)
 // int16 -> float without the int-to-float conversion unit: flipping the sign bit of q gives q + 32768 in
@@ -144,72 +146,63 @@ template <> struct LinkBytes<0> { static constexpr int v = 144; };
 template <> struct LinkBytes<1> { static constexpr int v = 72; };
 template <> struct LinkBytes<2> { static constexpr int v = 36; };
 
-template <int P>
+template <int P, bool KEEP = false>
 __device__ __forceinline__ void ld_link(const void *par_base, int pv, int dir, int i, float scale,
-                                        typename Acc<P>::T u[18]);
-
-template <> __device__ __forceinline__ void ld_link<0>(const void *par_base, int pv, int dir, int i, float scale,
-                                                       double u[18])
+                                        typename Acc<P>::T u[18])
 {
     (void)scale;
-    const double2 *b = static_cast<const double2 *>(par_base) + (size_t)dir * 9 * pv + i;
+    if constexpr (P == 0) {
+        const double2 *b = static_cast<const double2 *>(par_base) + (size_t)dir * 9 * pv + i;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        const double2 w = ld_stream(b + (size_t)k * pv);
-        u[2 * k] = w.x;
-        u[2 * k + 1] = w.y;
-    }
-}
-
-template <> __device__ __forceinline__ void ld_link<1>(const void *par_base, int pv, int dir, int i, float scale,
-                                                       float u[18])
-{
-    (void)scale;
-    const char *d = static_cast<const char *>(par_base) + (size_t)dir * 72 * pv;
-    const float4 *b4 = reinterpret_cast<const float4 *>(d) + i;
+        for (int k = 0; k < 9; ++k) {
+            const double2 w = ld_stream<KEEP>(b + (size_t)k * pv);
+            u[2 * k] = w.x;
+            u[2 * k + 1] = w.y;
+        }
+    } else if constexpr (P == 1) {
+        const char *d = static_cast<const char *>(par_base) + (size_t)dir * 72 * pv;
+        const float4 *b4 = reinterpret_cast<const float4 *>(d) + i;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float4 w = ld_stream(b4 + (size_t)k * pv);
-        u[4 * k] = w.x; u[4 * k + 1] = w.y; u[4 * k + 2] = w.z; u[4 * k + 3] = w.w;
-    }
-    const float2 w = ld_stream(reinterpret_cast<const float2 *>(d + (size_t)64 * pv) + i);
-    u[16] = w.x;
-    u[17] = w.y;
-}
-
-template <> __device__ __forceinline__ void ld_link<2>(const void *par_base, int pv, int dir, int i, float scale,
-                                                       float u[18])
-{
-    const char *d = static_cast<const char *>(par_base) + (size_t)dir * 36 * pv;
-    const int4 *b4 = reinterpret_cast<const int4 *>(d) + i;
-    const float s = scale * (1.0f / 32767.0f);
+        for (int k = 0; k < 4; ++k) {
+            const float4 w = ld_stream<KEEP>(b4 + (size_t)k * pv);
+            u[4 * k] = w.x; u[4 * k + 1] = w.y; u[4 * k + 2] = w.z; u[4 * k + 3] = w.w;
+        }
+        const float2 w = ld_stream<KEEP>(reinterpret_cast<const float2 *>(d + (size_t)64 * pv) + i);
+        u[16] = w.x;
+        u[17] = w.y;
+    } else {
+        const char *d = static_cast<const char *>(par_base) + (size_t)dir * 36 * pv;
+        const int4 *b4 = reinterpret_cast<const int4 *>(d) + i;
+        const float s = scale * (1.0f / 32767.0f);
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int4 w = ld_stream(b4 + (size_t)k * pv);
-        u[8 * k + 0] = lo16(w.x) * s; u[8 * k + 1] = hi16(w.x) * s;
-        u[8 * k + 2] = lo16(w.y) * s; u[8 * k + 3] = hi16(w.y) * s;
-        u[8 * k + 4] = lo16(w.z) * s; u[8 * k + 5] = hi16(w.z) * s;
-        u[8 * k + 6] = lo16(w.w) * s; u[8 * k + 7] = hi16(w.w) * s;
+        for (int k = 0; k < 2; ++k) {
+            const int4 w = ld_stream<KEEP>(b4 + (size_t)k * pv);
+            u[8 * k + 0] = lo16(w.x) * s; u[8 * k + 1] = hi16(w.x) * s;
+            u[8 * k + 2] = lo16(w.y) * s; u[8 * k + 3] = hi16(w.y) * s;
+            u[8 * k + 4] = lo16(w.z) * s; u[8 * k + 5] = hi16(w.z) * s;
+            u[8 * k + 6] = lo16(w.w) * s; u[8 * k + 7] = hi16(w.w) * s;
+        }
+        const int w = ld_stream<KEEP>(reinterpret_cast<const int *>(d + (size_t)32 * pv) + i);
+        u[16] = lo16(w) * s;
+        u[17] = hi16(w) * s;
     }
-    const int w = ld_stream(reinterpret_cast<const int *>(d + (size_t)32 * pv) + i);
-    u[16] = lo16(w) * s;
-    u[17] = hi16(w) * s;
 }
 
 // HALF link as raw int16 values (the per-field scale is applied by the caller, once per site)
+template <bool KEEP = false>
 __device__ __forceinline__ void ld_link_q16(const void *par_base, int pv, int dir, int i, float u[18])
 {
     const char *d = static_cast<const char *>(par_base) + (size_t)dir * 36 * pv;
     const int4 *b4 = reinterpret_cast<const int4 *>(d) + i;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        const int4 w = ld_stream(b4 + (size_t)k * pv);
+        const int4 w = ld_stream<KEEP>(b4 + (size_t)k * pv);
         u[8 * k + 0] = lo16(w.x); u[8 * k + 1] = hi16(w.x);
         u[8 * k + 2] = lo16(w.y); u[8 * k + 3] = hi16(w.y);
         u[8 * k + 4] = lo16(w.z); u[8 * k + 5] = hi16(w.z);
         u[8 * k + 6] = lo16(w.w); u[8 * k + 7] = hi16(w.w);
     }
-    const int w = ld_stream(reinterpret_cast<const int *>(d + (size_t)32 * pv) + i);
+    const int w = ld_stream<KEEP>(reinterpret_cast<const int *>(d + (size_t)32 * pv) + i);
     u[16] = lo16(w);
     u[17] = hi16(w);
 }
@@ -272,48 +265,41 @@ __device__ __forceinline__ void rebuild_row2(T u[18], T inv_s)
     }
 }
 
-template <int P>
-__device__ __forceinline__ void ld_link_recon(const void *par_base, int pv, int dir, int i,
-                                              typename Acc<P>::T u[18]);
-
-template <> __device__ __forceinline__ void ld_link_recon<0>(const void *par_base, int pv, int dir, int i, double u[18])
+template <int P, bool KEEP = false>
+__device__ __forceinline__ void ld_link_recon(const void *par_base, int pv, int dir, int i, typename Acc<P>::T u[18])
 {
-    const char *d = static_cast<const char *>(par_base) + (size_t)dir * 104 * pv;
-    const double2 *b = reinterpret_cast<const double2 *>(d) + i;
+    if constexpr (P == 0) {
+        const char *d = static_cast<const char *>(par_base) + (size_t)dir * 104 * pv;
+        const double2 *b = reinterpret_cast<const double2 *>(d) + i;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const double2 w = ld_stream(b + (size_t)k * pv);
-        u[2 * k] = w.x;
-        u[2 * k + 1] = w.y;
+        for (int k = 0; k < 6; ++k) {
+            const double2 w = ld_stream<KEEP>(b + (size_t)k * pv);
+            u[2 * k] = w.x;
+            u[2 * k + 1] = w.y;
+        }
+        rebuild_row2(u, ld_stream<KEEP>(reinterpret_cast<const double *>(d + (size_t)96 * pv) + i));
+    } else if constexpr (P == 1) {
+        const char *d = static_cast<const char *>(par_base) + (size_t)dir * 52 * pv;
+        const float4 *b4 = reinterpret_cast<const float4 *>(d) + i;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float4 w = ld_stream<KEEP>(b4 + (size_t)k * pv);
+            u[4 * k] = w.x; u[4 * k + 1] = w.y; u[4 * k + 2] = w.z; u[4 * k + 3] = w.w;
+        }
+        rebuild_row2(u, ld_stream<KEEP>(reinterpret_cast<const float *>(d + (size_t)48 * pv) + i));
+    } else {
+#pragma unroll
+        for (int k = 0; k < 18; ++k) u[k] = 0.f;  // HALF links are never stored compressed
     }
-    rebuild_row2(u, __ldcs(reinterpret_cast<const double *>(d + (size_t)96 * pv) + i));
-}
-
-template <> __device__ __forceinline__ void ld_link_recon<1>(const void *par_base, int pv, int dir, int i, float u[18])
-{
-    const char *d = static_cast<const char *>(par_base) + (size_t)dir * 52 * pv;
-    const float4 *b4 = reinterpret_cast<const float4 *>(d) + i;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float4 w = ld_stream(b4 + (size_t)k * pv);
-        u[4 * k] = w.x; u[4 * k + 1] = w.y; u[4 * k + 2] = w.z; u[4 * k + 3] = w.w;
-    }
-    rebuild_row2(u, __ldcs(reinterpret_cast<const float *>(d + (size_t)48 * pv) + i));
-}
-
-template <> __device__ __forceinline__ void ld_link_recon<2>(const void *, int, int, int, float u[18])
-{
-#pragma unroll
-    for (int k = 0; k < 18; ++k) u[k] = 0.f;  // HALF links are never stored compressed
 }
 
 // any storage of a LinkSet: full (recon = 0) or compressed
-template <int P>
+template <int P, bool KEEP = false>
 __device__ __forceinline__ void ld_link_any(const void *par_base, int pv, int dir, int i, float scale, int recon,
                                             typename Acc<P>::T u[18])
 {
-    if (P != 2 && recon) ld_link_recon<P>(par_base, pv, dir, i, u);
-    else ld_link<P>(par_base, pv, dir, i, scale, u);
+    if (P != 2 && recon) ld_link_recon<P, KEEP>(par_base, pv, dir, i, u);
+    else ld_link<P, KEEP>(par_base, pv, dir, i, scale, u);
 }
 
 // store rows 0, 1 and inv_s of one link in the compressed layout
