@@ -443,8 +443,9 @@ KQ_API KuQCDStatus kq_true_residuals(kq_context *ctx, int parity, int num_shift,
     cudaSetDevice(ctx->device);
     const size_t vb = spinor_bytes(ctx->g, P64);
     const size_t pb = resid_partials_bytes(ctx->g, num_shift), sb = sizeof(double) * (kMaxShift + 1);
-    // temporaries for eight shifts at a time, or for the four that share a link load
-    int fields = std::min(num_shift, 8);
+    // temporaries for sixteen shifts at a time (24^3 x 48, 12 shifts: 1.03 ms, eight at a time 1.11 ms), or for the four
+    // that share a link load
+    int fields = std::min(num_shift, 16);
     auto bytes = [&] {
         Carve c(nullptr);
         c.take(vb * fields);
