@@ -205,8 +205,9 @@ def run_lattice(cfg, args, rank, world, local, steps, warmup, plain_steps, e2e_s
 
     def solver_kw(name):
         if name in ("fp64", "fp64w"):
-            # plain CGM stopping rule tol = (rel * |b|)^2 on the recursive residual of every shift; "fp64" keeps the
-            # reference's kernel order, "fp64w" defers the shift updates over windows of 16 iterations
+            # plain CGM stopping rule tol = (rel * |b|)^2 on the recursive residual of every shift; both defer the shift
+            # updates over windows of 16 iterations ("fp64" goes back to the reference's kernel order where the device
+            # has no room for the ring of residuals)
             return dict(parity=0, solver=K.KQ_SOLVER_CGM if name == "fp64" else K.KQ_SOLVER_CGM_WINDOWED,
                         prec=K.KUQCD_DOUBLE, max_iter=100000, tol=(REL_RES ** 2) * bnorm2, shift_mode=1)
         return dict(parity=0, solver=K.KQ_SOLVER_MIXED, prec=sloppy[name], max_iter=100000, rel_residual=REL_RES,

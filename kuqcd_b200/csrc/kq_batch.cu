@@ -8,7 +8,8 @@
 //
 // Each system runs the windowed multishift CG of kq_msrelax.cu (the CGM recurrences of inverter_cgm.cpp:17-87,
 // deferred shift updates, operator precision relaxed FP64 -> FP32 -> HALF as its own residual falls -- decided on
-// the device per system, kq_ms_device.cuh).  Reductions are per system: every tile publishes a partial sum and
+// the device per system, kq_ms_device.cuh, and applied at the end of a chunk of iterations, so that the host enqueues
+// only the kernels of the precisions in use).  Reductions are per system: every tile publishes a partial sum and
 // the CTA that completes a system's last tile (per-system atomic ticket) runs that system's scalar step.
 // After the batched phase every system gets the FP64 true-residual check (and, if needed, the refinement) of the
 // single-system mixed solver.

@@ -131,7 +131,7 @@ int resid_tiles(const Geom &g) { return (g.vh + kBSr - 1) / kBSr; }
 size_t resid_partials_bytes(const Geom &g, int ns) { return sizeof(double) * (size_t)resid_tiles(g) * (ns + 1); }
 
 // |b - (sigma_k - D D) x_k|^2 for every k and |b|^2 of one parity: sums[0 .. ns - 1], sums[ns] on the host (pinned).
-// x fields xstride bytes apart; tmp holds `fields` >= min(ns, 4) of them, so at most that many shifts go in a launch.
+// x fields xstride bytes apart; tmp holds `fields` >= 1 of them, so at most that many shifts go in a launch.
 cudaError_t residual_norms(const Geom &g, const GaugeDev &gd, int parity, int ns, const double *sigma, const void *d_b,
                            const void *d_x, size_t xstride, void *tmp, int fields, double *partials, double *d_sums,
                            double *sums, cudaStream_t s)
@@ -142,7 +142,8 @@ cudaError_t residual_norms(const Geom &g, const GaugeDev &gd, int parity, int ns
     for (int k = 0; k < ns; ++k) sg.v[k] = sigma[k];
     // one solution per thread while all of them fit one wave (8^4, 12 shifts: 10.6 us per half, four per thread 14.6 us;
     // 16^4: 80.8 and 46.4 us); the links then come from the L2
-    const int most = (long long)g.vh * ns <= 148 * 3 * 256 ? 1 : 4;
+    const int fit = fields < 4 ? fields : 4;
+    const int most = (long long)g.vh * ns <= 148 * 3 * 256 ? 1 : fit;
     const int groups = (ns + most - 1) / most, base = ns / groups, larger = ns % groups;  // `larger` groups of base + 1
     int k0 = 0;
     for (int part = 0; part < 2; ++part) {

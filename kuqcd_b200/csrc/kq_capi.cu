@@ -443,8 +443,7 @@ KQ_API KuQCDStatus kq_true_residuals(kq_context *ctx, int parity, int num_shift,
     cudaSetDevice(ctx->device);
     const size_t vb = spinor_bytes(ctx->g, P64);
     const size_t pb = resid_partials_bytes(ctx->g, num_shift), sb = sizeof(double) * (kMaxShift + 1);
-    // temporaries for sixteen shifts at a time (24^3 x 48, 12 shifts: 1.03 ms, eight at a time 1.11 ms), or for the four
-    // that share a link load
+    // temporaries for sixteen shifts at a time (24^3 x 48, 12 shifts: 1.03 ms, eight at a time 1.11 ms)
     int fields = std::min(num_shift, 16);
     auto bytes = [&] {
         Carve c(nullptr);
@@ -454,9 +453,10 @@ KQ_API KuQCDStatus kq_true_residuals(kq_context *ctx, int parity, int num_shift,
         return c.off;
     };
     cudaError_t e = ensure_work(ctx, bytes());
-    if (e == cudaErrorMemoryAllocation && fields > 4) {
+    while (e == cudaErrorMemoryAllocation && fields > 1) {  // as many as the device has room for
         cudaGetLastError();
-        fields = 4;
+        fields /= 4;
+        if (fields < 1) fields = 1;
         e = ensure_work(ctx, bytes());
     }
     if (e != cudaSuccess) return status_of(e);
