@@ -93,6 +93,13 @@ struct CgmState;
 cudaError_t launch_dslash_axmy_dot(const Geom &g, const GaugeDev &gd, int prec, const void *tmp, const void *p,
                                    void *s_out, int parity, CgmState *st, cudaStream_t s);
 
+// Grid of a kernel over tiles of `block` sites times ng groups of systems, block x = tile * ng + group.  On x alone: a
+// context's 2^31 sites in tiles of 128, times the 16 groups of 64 systems, are 2^28 blocks of the 2^31 - 1 allowed there.
+inline dim3 tile_group_grid(int sites, int block, int ng)
+{
+    return dim3((unsigned)((sites + (long long)block - 1) / block) * (unsigned)ng);
+}
+
 // Launch with programmatic stream serialization: the kernel may start while the one before it in the stream ends (both
 // use pdl_trigger / pdl_wait of kq_dslash_core.cuh).
 template <typename... P, typename... A>

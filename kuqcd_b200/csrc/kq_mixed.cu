@@ -65,6 +65,17 @@ __device__ __forceinline__ void group_systems(const int *list, int n, int grp, i
     }
 }
 
+// Tile of sites and group of systems of this block.  A tile's groups are neighbours in the grid, so that all but the
+// first find its links in the L2.  Everything is on x (tile_group_grid): the y extent of a grid ends at 65,535, which
+// tiles of 128 sites reach at 64^4.
+struct MrTile {
+    int grp, tile, ntiles;
+    __device__ __forceinline__ explicit MrTile(int ng)
+        : grp(blockIdx.x % ng), tile(blockIdx.x / ng), ntiles(gridDim.x / ng)
+    {
+    }
+};
+
 // true in every thread of the last block of the grid to finish (after all others published their partials)
 __device__ __forceinline__ bool last_block(unsigned *ticket)
 {
@@ -73,7 +84,7 @@ __device__ __forceinline__ bool last_block(unsigned *ticket)
     if (threadIdx.x == 0) {
         __threadfence();
         const unsigned t = atomicAdd(ticket, 1u);
-        last = (t == gridDim.x * gridDim.y - 1);
+        last = (t == gridDim.x - 1);
     }
     __syncthreads();
     if (last) __threadfence();
@@ -84,12 +95,13 @@ __device__ __forceinline__ bool last_block(unsigned *ticket)
 // K1: tmp_k = D p_k (output parity q) for the active systems
 template <int LP, int R>
 __global__ void __launch_bounds__(kBS) mr_dslash_kernel(Geom g, int pv, LinkSet fat, LinkSet lng, const char *p0,
-                                                        char *tmp0, size_t vb, int q, const MrState *st)
+                                                        char *tmp0, size_t vb, int q, const MrState *st, int ng)
 {
+    const MrTile w(ng);
     int sys[R];
-    group_systems<R>(st->act, st->nact, blockIdx.x, sys);
+    group_systems<R>(st->act, st->nact, w.grp, sys);
     if (sys[0] < 0) return;
-    const int i = blockIdx.y * kBS + threadIdx.x;
+    const int i = w.tile * kBS + threadIdx.x;
     if (i >= g.vh) return;
     float acc[R][6];
     dslash_site_mrhs<LP, 1, R>(g, pv, fat, lng, p0, vb, sys, q, i, acc);
@@ -102,13 +114,14 @@ __global__ void __launch_bounds__(kBS) mr_dslash_kernel(Geom g, int pv, LinkSet 
 template <int LP, int R>
 __global__ void __launch_bounds__(kBS) mr_dslash2_kernel(Geom g, int pv, LinkSet fat, LinkSet lng, const char *tmp0,
                                                          const char *p0, char *ap0, size_t vb, int parity, MrState *st,
-                                                         double *partials)
+                                                         double *partials, int ng)
 {
+    const MrTile w(ng);
     __shared__ double sm[32];
     int sys[R];
     const int n = st->nact;
-    group_systems<R>(st->act, n, blockIdx.x, sys);
-    const int i = blockIdx.y * kBS + threadIdx.x;
+    group_systems<R>(st->act, n, w.grp, sys);
+    const int i = w.tile * kBS + threadIdx.x;
     double dot[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) dot[r] = 0.0;
@@ -132,12 +145,12 @@ __global__ void __launch_bounds__(kBS) mr_dslash2_kernel(Geom g, int pv, LinkSet
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const double s = block_sum(dot[r], sm);
-        if (threadIdx.x == 0 && sys[r] >= 0) partials[sys[r] * gridDim.y + blockIdx.y] = s;
+        if (threadIdx.x == 0 && sys[r] >= 0) partials[(size_t)sys[r] * w.ntiles + w.tile] = s;
     }
     if (!last_block(&st->ticket[0])) return;
     for (int a = 0; a < n; ++a) {
         const int k = st->act[a];
-        const double pAp = partials_sum(partials + (size_t)k * gridDim.y, gridDim.y, sm);
+        const double pAp = partials_sum(partials + (size_t)k * w.ntiles, w.ntiles, sm);
         if (threadIdx.x == 0) st->alpha[k] = st->rr[k] / pAp;
     }
     if (threadIdx.x == 0) st->ticket[0] = 0;
@@ -146,13 +159,14 @@ __global__ void __launch_bounds__(kBS) mr_dslash2_kernel(Geom g, int pv, LinkSet
 // K3: xs_k += alpha_k p_k ; r_k -= alpha_k ap_k ; |r_k|^2 -> reliable-update decision or beta_k
 template <int R>
 __global__ void __launch_bounds__(kBS) mr_update_kernel(int vh, int pv, const char *p0, const char *ap0, char *r0,
-                                                        char *xs0, size_t vb, MrState *st, double *partials)
+                                                        char *xs0, size_t vb, MrState *st, double *partials, int ng)
 {
+    const MrTile w(ng);
     __shared__ double sm[32];
     int sys[R];
     const int n = st->nact;
-    group_systems<R>(st->act, n, blockIdx.x, sys);
-    const int i = blockIdx.y * kBS + threadIdx.x;
+    group_systems<R>(st->act, n, w.grp, sys);
+    const int i = w.tile * kBS + threadIdx.x;
     double nn[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) nn[r] = 0.0;
@@ -180,7 +194,7 @@ __global__ void __launch_bounds__(kBS) mr_update_kernel(int vh, int pv, const ch
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const double s = block_sum(nn[r], sm);
-        if (threadIdx.x == 0 && sys[r] >= 0) partials[sys[r] * gridDim.y + blockIdx.y] = s;
+        if (threadIdx.x == 0 && sys[r] >= 0) partials[(size_t)sys[r] * w.ntiles + w.tile] = s;
     }
     if (!last_block(&st->ticket[1])) return;
     __shared__ int nflag;
@@ -188,7 +202,7 @@ __global__ void __launch_bounds__(kBS) mr_update_kernel(int vh, int pv, const ch
     __syncthreads();
     for (int a = 0; a < n; ++a) {
         const int k = st->act[a];
-        const double rr = partials_sum(partials + (size_t)k * gridDim.y, gridDim.y, sm);
+        const double rr = partials_sum(partials + (size_t)k * w.ntiles, w.ntiles, sm);
         if (threadIdx.x == 0) {
             st->sys_iter[k] += 1;
             if (rr < st->target2 || rr < st->delta2 * st->maxrr[k] || !isfinite(rr)) {
@@ -208,12 +222,13 @@ __global__ void __launch_bounds__(kBS) mr_update_kernel(int vh, int pv, const ch
 // K4: x64_k += xs_k ; xs_k = 0  (flagged systems)
 template <int R>
 __global__ void __launch_bounds__(kBS) mr_accum_kernel(int vh, int pv, char *xs0, size_t vb, char *x640,
-                                                       size_t vb64, const MrState *st)
+                                                       size_t vb64, const MrState *st, int ng)
 {
+    const MrTile w(ng);
     int sys[R];
-    group_systems<R>(st->flag, st->nflag, blockIdx.x, sys);
+    group_systems<R>(st->flag, st->nflag, w.grp, sys);
     if (sys[0] < 0) return;
-    const int i = blockIdx.y * kBS + threadIdx.x;
+    const int i = w.tile * kBS + threadIdx.x;
     if (i >= vh) return;
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -236,12 +251,13 @@ __global__ void __launch_bounds__(kBS) mr_accum_kernel(int vh, int pv, char *xs0
 // K5: tmp64_k = D x64_k (FP64, flagged systems, output parity q)
 template <int R>
 __global__ void __launch_bounds__(kBS64, kCtas64) mr_dslash64_kernel(Geom g, int pv, LinkSet fat, LinkSet lng, const char *x640,
-                                                          char *t640, size_t vb64, int q, const MrState *st)
+                                                          char *t640, size_t vb64, int q, const MrState *st, int ng)
 {
+    const MrTile w(ng);
     int sys[R];
-    group_systems<R>(st->flag, st->nflag, blockIdx.x, sys);
+    group_systems<R>(st->flag, st->nflag, w.grp, sys);
     if (sys[0] < 0) return;
-    const int i = blockIdx.y * kBS64 + threadIdx.x;
+    const int i = w.tile * kBS64 + threadIdx.x;
     if (i >= g.vh) return;
     double acc[R][6];
     if (sys[R - 1] >= 0) dslash_site_mrhs<0, 0, R, true>(g, pv, fat, lng, x640, vb64, sys, q, i, acc);
@@ -255,14 +271,15 @@ __global__ void __launch_bounds__(kBS64, kCtas64) mr_dslash64_kernel(Geom g, int
 template <int R>
 __global__ void __launch_bounds__(kBS64, kCtas64) mr_resid_kernel(Geom g, int pv, LinkSet fat, LinkSet lng, const char *t640,
                                                        const char *x640, size_t vb64, const void *b, char *r0,
-                                                       size_t vb, int parity, MrState *st, double *partials)
+                                                       size_t vb, int parity, MrState *st, double *partials, int ng)
 {
+    const MrTile w(ng);
     __shared__ double sm[32];
     const int n = st->nflag;
     if (n == 0) return;
     int sys[R];
-    group_systems<R>(st->flag, n, blockIdx.x, sys);
-    const int i = blockIdx.y * kBS64 + threadIdx.x;
+    group_systems<R>(st->flag, n, w.grp, sys);
+    const int i = w.tile * kBS64 + threadIdx.x;
     double nn[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) nn[r] = 0.0;
@@ -291,12 +308,12 @@ __global__ void __launch_bounds__(kBS64, kCtas64) mr_resid_kernel(Geom g, int pv
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const double s = block_sum(nn[r], sm);
-        if (threadIdx.x == 0 && sys[r] >= 0) partials[sys[r] * gridDim.y + blockIdx.y] = s;
+        if (threadIdx.x == 0 && sys[r] >= 0) partials[(size_t)sys[r] * w.ntiles + w.tile] = s;
     }
     if (!last_block(&st->ticket[2])) return;
     for (int a = 0; a < n; ++a) {
         const int k = st->flag[a];
-        const double rr = partials_sum(partials + (size_t)k * gridDim.y, gridDim.y, sm);
+        const double rr = partials_sum(partials + (size_t)k * w.ntiles, w.ntiles, sm);
         if (threadIdx.x == 0) {
             const double rel = sqrt(rr / st->bnorm2);
             st->res[k] = rel;
@@ -319,12 +336,14 @@ __global__ void __launch_bounds__(kBS64, kCtas64) mr_resid_kernel(Geom g, int pv
 
 // K7: p_k = r_k + beta_k p_k for active, unconverged systems ; compaction of the active list
 template <int R>
-__global__ void __launch_bounds__(kBS) mr_p_kernel(int vh, int pv, const char *r0, char *p0, size_t vb, MrState *st)
+__global__ void __launch_bounds__(kBS) mr_p_kernel(int vh, int pv, const char *r0, char *p0, size_t vb, MrState *st,
+                                                   int ng)
 {
+    const MrTile w(ng);
     int sys[R];
     const int n = st->nact;
-    group_systems<R>(st->act, n, blockIdx.x, sys);
-    const int i = blockIdx.y * kBS + threadIdx.x;
+    group_systems<R>(st->act, n, w.grp, sys);
+    const int i = w.tile * kBS + threadIdx.x;
     if (i < vh) {
 #pragma unroll
         for (int r = 0; r < R; ++r)
@@ -378,29 +397,30 @@ constexpr int kR = 4;    // systems per thread in the sloppy multi-RHS kernels
 template <int LP>
 static void enqueue_reliable(const Geom &g, const GaugeDev &gd, const MrBuffers &w, int parity, int ns, cudaStream_t s)
 {
-    const int pv = pad_sites(g.vh), sb = (g.vh + kBS - 1) / kBS;
-    const dim3 g64((ns + kR64 - 1) / kR64, (g.vh + kBS64 - 1) / kBS64), gs((ns + kR - 1) / kR, sb);
-    mr_accum_kernel<kR><<<gs, kBS, 0, s>>>(g.vh, pv, (char *)w.xs, w.vb32, (char *)w.x64, w.vb64, w.st);
+    const int pv = pad_sites(g.vh), ng = (ns + kR - 1) / kR, ng64 = (ns + kR64 - 1) / kR64;
+    const dim3 g64 = tile_group_grid(g.vh, kBS64, ng64), gs = tile_group_grid(g.vh, kBS, ng);
+    mr_accum_kernel<kR><<<gs, kBS, 0, s>>>(g.vh, pv, (char *)w.xs, w.vb32, (char *)w.x64, w.vb64, w.st, ng);
     mr_dslash64_kernel<kR64><<<g64, kBS64, 0, s>>>(g, pv, gd.fat[0], gd.lng[0], (const char *)w.x64, (char *)w.tmp64,
-                                                 w.vb64, 1 - parity, w.st);
+                                                 w.vb64, 1 - parity, w.st, ng64);
     mr_resid_kernel<kR64><<<g64, kBS64, 0, s>>>(g, pv, gd.fat[0], gd.lng[0], (const char *)w.tmp64,
                                               (const char *)w.x64, w.vb64, w.b, (char *)w.r, w.vb32, parity, w.st,
-                                              w.partials);
-    mr_p_kernel<kR><<<gs, kBS, 0, s>>>(g.vh, pv, (const char *)w.r, (char *)w.p, w.vb32, w.st);
+                                              w.partials, ng64);
+    mr_p_kernel<kR><<<gs, kBS, 0, s>>>(g.vh, pv, (const char *)w.r, (char *)w.p, w.vb32, w.st, ng);
 }
 
 template <int LP>
 static void enqueue_mr_iteration(const Geom &g, const GaugeDev &gd, const MrBuffers &w, int parity, int ns,
                                  cudaStream_t s)
 {
-    const int pv = pad_sites(g.vh), sb = (g.vh + kBS - 1) / kBS;
-    const dim3 gs((ns + kR - 1) / kR, sb);
+    const int pv = pad_sites(g.vh), ng = (ns + kR - 1) / kR;
+    const dim3 gs = tile_group_grid(g.vh, kBS, ng);
     mr_dslash_kernel<LP, kR><<<gs, kBS, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], (const char *)w.p, (char *)w.tmp,
-                                                w.vb32, 1 - parity, w.st);
+                                                w.vb32, 1 - parity, w.st, ng);
     mr_dslash2_kernel<LP, kR><<<gs, kBS, 0, s>>>(g, pv, gd.fat[LP], gd.lng[LP], (const char *)w.tmp,
-                                                 (const char *)w.p, (char *)w.ap, w.vb32, parity, w.st, w.partials);
+                                                 (const char *)w.p, (char *)w.ap, w.vb32, parity, w.st, w.partials,
+                                                 ng);
     mr_update_kernel<kR><<<gs, kBS, 0, s>>>(g.vh, pv, (const char *)w.p, (const char *)w.ap, (char *)w.r,
-                                            (char *)w.xs, w.vb32, w.st, w.partials);
+                                            (char *)w.xs, w.vb32, w.st, w.partials, ng);
     enqueue_reliable<LP>(g, gd, w, parity, ns, s);
 }
 
