@@ -45,13 +45,36 @@ cudaError_t ensure_work(::kq_context *ctx, size_t bytes)
     if (ctx->work_bytes >= bytes) return cudaSuccess;
     if (ctx->work) {
         KQ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        cudaFree(ctx->work);
-        ctx->work = nullptr;
-        ctx->work_bytes = 0;
+        release_work(ctx);
     }
     KQ_CUDA_TRY(cudaMalloc(&ctx->work, bytes));
     ctx->work_bytes = bytes;
     return cudaSuccess;
+}
+
+void release_work(::kq_context *ctx)
+{
+    if (ctx->work) cudaFree(ctx->work);
+    ctx->work = nullptr;
+    ctx->work_bytes = 0;
+}
+
+bool optional_work(::kq_context *ctx, size_t want, int share)
+{
+    if (ctx->work_bytes >= want) return true;
+    const size_t have = ctx->work_bytes;
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (!ctx->work_policy.may_grow(want, have, free, share)) return false;
+    const std::string text = last_error();
+    if (ensure_work(ctx, want) == cudaSuccess) return true;
+    cudaGetLastError();
+    set_last_error(text);
+    ctx->work_policy.note_failure(want, have, free);
+    return false;
 }
 
 static cudaError_t alloc_links(::kq_context *ctx, int prec)
@@ -443,7 +466,8 @@ KQ_API KuQCDStatus kq_true_residuals(kq_context *ctx, int parity, int num_shift,
     cudaSetDevice(ctx->device);
     const size_t vb = spinor_bytes(ctx->g, P64);
     const size_t pb = resid_partials_bytes(ctx->g, num_shift), sb = sizeof(double) * (kMaxShift + 1);
-    // temporaries for sixteen shifts at a time (24^3 x 48, 12 shifts: 1.03 ms, eight at a time 1.11 ms)
+    // temporaries for sixteen shifts at a time (24^3 x 48, 12 shifts: 1.03 ms, eight at a time 1.11 ms) as far as they
+    // fit the workspace there is or 512 MiB, and two where nothing else does (48^3 x 96: 510 MB)
     int fields = std::min(num_shift, 16);
     auto bytes = [&] {
         Carve c(nullptr);
@@ -452,13 +476,10 @@ KQ_API KuQCDStatus kq_true_residuals(kq_context *ctx, int parity, int num_shift,
         c.take(sb);
         return c.off;
     };
+    while (fields > 2 && bytes() > WorkPolicy::budget(ctx->work_bytes)) --fields;
+    // fewer where the device has no room for that many
+    while (fields > 1 && !optional_work(ctx, bytes(), fields > 2 ? 4 : 1)) fields = fields > 4 ? 4 : fields > 2 ? 2 : 1;
     cudaError_t e = ensure_work(ctx, bytes());
-    while (e == cudaErrorMemoryAllocation && fields > 1) {  // as many as the device has room for
-        cudaGetLastError();
-        fields /= 4;
-        if (fields < 1) fields = 1;
-        e = ensure_work(ctx, bytes());
-    }
     if (e != cudaSuccess) return status_of(e);
     Carve w(ctx->work);
     void *tmp = w.take(vb * fields);
@@ -481,14 +502,6 @@ KQ_API KuQCDStatus kq_true_residuals(kq_context *ctx, int parity, int num_shift,
 
 static KuQCDStatus solve_full(kq_context *ctx, const kq_solve_param *p, const void *d_b, void *d_x,
                               kq_solve_info *info);
-
-// whether the workspace of the windowed solver is there or could be allocated
-static bool windowed_work(kq_context *ctx, int num_shift)
-{
-    if (ensure_work(ctx, ms_workspace_bytes(ctx->g, num_shift)) == cudaSuccess) return true;
-    cudaGetLastError();  // the caller goes on without it
-    return false;
-}
 
 // multishift CG with windowed shift updates, all in FP64 (kq_msrelax.cu)
 static cudaError_t windowed_solve(kq_context *ctx, const kq_solve_param *p, const double *sig, const void *d_b,
@@ -526,6 +539,8 @@ KQ_API KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_pa
     memset(info, 0, sizeof(*info));
     info->num_shift = p->num_shift;
 
+    const size_t work_before = ctx->work_bytes;
+    size_t work_need = 0;  // what the call can do with, where that is less than what it takes
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -547,10 +562,34 @@ KQ_API KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_pa
         }
         // In FP64 the windowed solver takes the same steps with (4 N + 16) / 16 instead of 4 N vector passes per
         // iteration for N shifts and three kernels instead of four: 24^3 x 48, 12 shifts, 0.303 ms per iteration in
-        // the reference's kernel order and 0.235 ms windowed.  It keeps a ring of 16 residuals; where the device
-        // has no room for that, and in FP32 (whose recurrences would lose digits in the window's products), the
-        // reference's kernel order remains.
-        if (prec == P64 && windowed_work(ctx, p->num_shift)) {
+        // the reference's kernel order and 0.235 ms windowed.  It takes a ring of 16 residuals; where that is more
+        // than a quarter of the device's free memory, and in FP32 (whose recurrences would lose digits in the
+        // window's products), the reference's kernel order remains.
+        const Geom &g = ctx->g;
+        const size_t vb = spinor_bytes(g, prec), vb64 = spinor_bytes(g, P64);
+        const int nb = (g.vh + 255) / 256;
+        const int ns = p->num_shift;
+        auto layout = [&](Carve &c, CgmBuffers &w) {
+            w.vec_bytes = vb;
+            w.r = c.take(vb);
+            w.s = c.take(vb);
+            w.tmp = c.take(vb);
+            w.p = c.take(vb * ns);
+            w.partials = static_cast<double *>(c.take(sizeof(double) * nb));
+            w.state = static_cast<CgmState *>(c.take(sizeof(CgmState)));
+            if (prec != P64) {
+                w.b = c.take(vb);
+                w.x = c.take(vb * ns);
+            } else {
+                w.b = d_b;
+                w.x = d_x;
+            }
+        };
+        CgmBuffers w;
+        Carve probe(nullptr);
+        layout(probe, w);
+        if (prec == P64 && optional_work(ctx, ms_workspace_bytes(g, ns), 4)) {
+            work_need = probe.off;
             // this solver reports no solution before its end
             auto *const ready = ctx->solution_ready;
             ctx->solution_ready = nullptr;
@@ -558,29 +597,6 @@ KQ_API KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_pa
             ctx->solution_ready = ready;
             if (e == cudaSuccess && info->status == 0 && info->iter >= p->max_iter) info->status = KQ_STATUS_MAXITER;
         } else {
-            const Geom &g = ctx->g;
-            const size_t vb = spinor_bytes(g, prec), vb64 = spinor_bytes(g, P64);
-            const int nb = (g.vh + 255) / 256;
-            const int ns = p->num_shift;
-            auto layout = [&](Carve &c, CgmBuffers &w) {
-                w.vec_bytes = vb;
-                w.r = c.take(vb);
-                w.s = c.take(vb);
-                w.tmp = c.take(vb);
-                w.p = c.take(vb * ns);
-                w.partials = static_cast<double *>(c.take(sizeof(double) * nb));
-                w.state = static_cast<CgmState *>(c.take(sizeof(CgmState)));
-                if (prec != P64) {
-                    w.b = c.take(vb);
-                    w.x = c.take(vb * ns);
-                } else {
-                    w.b = d_b;
-                    w.x = d_x;
-                }
-            };
-            CgmBuffers w;
-            Carve probe(nullptr);
-            layout(probe, w);
             e = ensure_work(ctx, probe.off);
             if (e != cudaSuccess) return status_of(e);
             Carve c(ctx->work);
@@ -611,6 +627,10 @@ KQ_API KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_pa
     info->seconds = ms * 1e-3;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    if (work_need && WorkPolicy::give_back(ctx->work_bytes, work_before, work_need)) {
+        cudaStreamSynchronize(ctx->stream);
+        release_work(ctx);
+    }
     if (e != cudaSuccess) {
         if (std::string(last_error()).empty()) set_last_error(cudaGetErrorString(e));
         return status_of(e);

@@ -2,6 +2,7 @@
 #pragma once
 #include "kq_internal.h"
 #include "kq_solver.h"
+#include "kq_work.h"
 
 struct kq_context {
     int device = 0;
@@ -12,9 +13,10 @@ struct kq_context {
     int master = -1;  // precision of the loaded links (P64 or P32)
     bool fat_loaded = false, long_loaded = false;
     unsigned *d_scratch = nullptr;
-    // solver workspace (grown on demand, never shrunk)
+    // solver workspace: grown on demand and kept; what a call took for speed alone is bounded (kq_work.h)
     void *work = nullptr;
     size_t work_bytes = 0;
+    kq::WorkPolicy work_policy;
     // device fields and host-record staging of kq_solve_multishift (host buffers in and out), grown on demand
     void *io = nullptr;
     size_t io_bytes = 0;
@@ -53,6 +55,10 @@ struct Carve {
 };
 
 cudaError_t ensure_work(::kq_context *ctx, size_t bytes);
+// whether the workspace holds `want` bytes or, under the context's policy, could be grown to them; a call for which
+// this is false goes on in less (last error and its text are as before)
+bool optional_work(::kq_context *ctx, size_t want, int share);
+void release_work(::kq_context *ctx);
 KuQCDStatus status_of(cudaError_t e);
 
 // KQ_SOLVER_MIXED on one context (kq_mixed.cu); shifts_abs are absolute.  With run_phase1 = false, d_x already

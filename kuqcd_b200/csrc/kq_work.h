@@ -1,0 +1,37 @@
+// When a context's workspace may be larger than a call needs (host code only).
+#pragma once
+#include <algorithm>
+#include <cstddef>
+
+namespace kq {
+
+// Workspace that calls keep for speed alone.  512 MiB is 0.3 % of a B200's memory and holds all that the solver and the
+// residual check ask for up to 32^4 with 12 shifts (378 MB more for the windowed solver, 302 MB of temporaries).
+constexpr size_t kWorkKeep = size_t(512) << 20;
+
+struct WorkPolicy {
+    size_t failed = 0, failed_room = 0;  // smallest size that could not be allocated, and the room there was then
+
+    // whether a workspace of `want` bytes may replace one of `have` bytes, `free` bytes of device memory being left,
+    // for a call that also runs in a smaller one; it may take 1 / share of the free memory
+    bool may_grow(size_t want, size_t have, size_t free, int share) const
+    {
+        if (want > have && want - have > free / share) return false;
+        return !(failed && want >= failed && have + free <= failed_room);
+    }
+
+    void note_failure(size_t want, size_t have, size_t free)
+    {
+        failed = want;
+        failed_room = have + free;
+    }
+
+    // whether a workspace of `now` bytes goes back to the device after a call that could have run in `need` bytes and
+    // began with a workspace of `before`
+    static bool give_back(size_t now, size_t before, size_t need) { return now > std::max(before, need) + kWorkKeep; }
+
+    // the most a call takes for speed alone, with a workspace of `have` bytes there already
+    static size_t budget(size_t have) { return std::max(have, kWorkKeep); }
+};
+
+}  // namespace kq
