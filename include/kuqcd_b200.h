@@ -187,12 +187,16 @@ KuQCDStatus kq_slab_cgm_poll(kq_context *ctx, const kq_slab_cgm_state *d_state, 
 
 /* ---------------------------------------------------------------- solver */
 enum {
-    KQ_SOLVER_CGM = 0,        /* multishift CG with the reference's recurrences (CGM::Invert), FP64 or FP32 */
+    KQ_SOLVER_CGM = 0,        /* multishift CG with the reference's recurrences (CGM::Invert), FP64 or FP32.  In FP64
+                                 with the shift updates of KQ_SOLVER_CGM_WINDOWED where the workspace for them may be
+                                 had (kq_set_workspace_limit), else, and in FP32, in the reference's kernel order.
+                                 Reports no solution before its end. */
     KQ_SOLVER_MIXED = 1,      /* relaxed-precision multishift (FP64 -> FP32 -> HALF operator as |r| falls) with an
                                  FP64 true-residual check and batched reliable-update refinement of any shift left
                                  above rel_residual; prec = SINGLE or HALF is the cheapest operator it may use */
-    KQ_SOLVER_CGM_WINDOWED = 2 /* the CGM recurrences in FP64 with windowed shift updates (same iterates as
-                                  KQ_SOLVER_CGM up to rounding, 4N -> (4N+8)/8 vector sweeps per iteration) */
+    KQ_SOLVER_CGM_WINDOWED = 2 /* the CGM recurrences in FP64 with shift updates deferred over windows of 16
+                                  iterations (same iterates up to rounding, 4N -> (4N+16)/16 vector sweeps per
+                                  iteration), solutions reported as they converge */
 };
 
 enum { KQ_PARITY_FULL = 2 };
@@ -239,6 +243,12 @@ KuQCDStatus kq_solve_multishift(kq_context *ctx, const kq_solve_param *param, co
  * that for KQ_PARITY_FULL). */
 KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_param *param, const void *d_b, void *d_x,
                                        kq_solve_info *info);
+/* The most bytes of workspace this context holds on the device where a call can do with less; a larger workspace held
+ * from earlier calls is freed.  0 (the default): calls take at most a quarter of the free memory for speed alone and
+ * keep at most 512 MiB of it.  What depends on it: KQ_SOLVER_CGM in FP64 (num_shift + 18 FP64 fields, or num_shift + 3
+ * in the reference's kernel order, 0.303 against 0.235 ms per iteration at 24^3 x 48 with 12 shifts) and
+ * kq_true_residuals (one field of one parity for each of up to 16 shifts at a time; without a limit at least two). */
+KuQCDStatus kq_set_workspace_limit(kq_context *ctx, size_t bytes);
 /* FP64 true relative residuals |b - (sigma_k - DD) x_k| / |b| of device FP64 fields (absolute sigmas; parity
  * KQ_PARITY_FULL: full-lattice fields, norms over both parities). */
 KuQCDStatus kq_true_residuals(kq_context *ctx, int parity, int num_shift, const double *sigma, const void *d_b,

@@ -293,6 +293,19 @@ KQ_API KuQCDStatus kq_prepare_links(kq_context *ctx, int prec)
     return KUQCD_SUCCESS;
 }
 
+KQ_API KuQCDStatus kq_set_workspace_limit(kq_context *ctx, size_t bytes)
+{
+    if (!ctx) return KUQCD_ERR_NULL_POINTER;
+    ctx->work_policy.limit = bytes;
+    if (bytes && ctx->work_bytes > bytes) {
+        cudaSetDevice(ctx->device);
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        release_work(ctx);
+        return status_of(e);
+    }
+    return KUQCD_SUCCESS;
+}
+
 KQ_API size_t kq_spinor_bytes(const kq_context *ctx, int prec)
 {
     const int p = prec_from_api(prec);
@@ -476,7 +489,8 @@ KQ_API KuQCDStatus kq_true_residuals(kq_context *ctx, int parity, int num_shift,
         c.take(sb);
         return c.off;
     };
-    while (fields > 2 && bytes() > WorkPolicy::budget(ctx->work_bytes)) --fields;
+    const int least = ctx->work_policy.limit ? 1 : 2;
+    while (fields > least && bytes() > ctx->work_policy.budget(ctx->work_bytes)) --fields;
     // fewer where the device has no room for that many
     while (fields > 1 && !optional_work(ctx, bytes(), fields > 2 ? 4 : 1)) fields = fields > 4 ? 4 : fields > 2 ? 2 : 1;
     cudaError_t e = ensure_work(ctx, bytes());
@@ -563,7 +577,7 @@ KQ_API KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_pa
         // In FP64 the windowed solver takes the same steps with (4 N + 16) / 16 instead of 4 N vector passes per
         // iteration for N shifts and three kernels instead of four: 24^3 x 48, 12 shifts, 0.303 ms per iteration in
         // the reference's kernel order and 0.235 ms windowed.  It takes a ring of 16 residuals; where that is more
-        // than a quarter of the device's free memory, and in FP32 (whose recurrences would lose digits in the
+        // than a quarter of the device's free memory or than the caller's limit, and in FP32 (whose recurrences would lose digits in the
         // window's products), the reference's kernel order remains.
         const Geom &g = ctx->g;
         const size_t vb = spinor_bytes(g, prec), vb64 = spinor_bytes(g, P64);
@@ -627,7 +641,7 @@ KQ_API KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_pa
     info->seconds = ms * 1e-3;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (work_need && WorkPolicy::give_back(ctx->work_bytes, work_before, work_need)) {
+    if (work_need && ctx->work_policy.give_back(ctx->work_bytes, work_before, work_need)) {
         cudaStreamSynchronize(ctx->stream);
         release_work(ctx);
     }

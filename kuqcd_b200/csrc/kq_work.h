@@ -7,15 +7,19 @@ namespace kq {
 
 // Workspace that calls keep for speed alone.  512 MiB is 0.3 % of a B200's memory and holds all that the solver and the
 // residual check ask for up to 32^4 with 12 shifts (378 MB more for the windowed solver, 302 MB of temporaries).
+// Beyond it a solve takes its workspace anew, 3.6 of 604 ms at 48^4, and a residual check in a context that has solved
+// nothing takes fewer shifts at a time, 9.0 against 8.3 ms there.
 constexpr size_t kWorkKeep = size_t(512) << 20;
 
 struct WorkPolicy {
-    size_t failed = 0, failed_room = 0;  // smallest size that could not be allocated, and the room there was then
+    size_t limit = 0;  // the caller's (kq_set_workspace_limit); 0: none
+    size_t failed = 0, failed_room = 0;  // size that last could not be allocated, and the room there was then
 
     // whether a workspace of `want` bytes may replace one of `have` bytes, `free` bytes of device memory being left,
     // for a call that also runs in a smaller one; it may take 1 / share of the free memory
     bool may_grow(size_t want, size_t have, size_t free, int share) const
     {
+        if (limit && want > limit) return false;
         if (want > have && want - have > free / share) return false;
         return !(failed && want >= failed && have + free <= failed_room);
     }
@@ -27,11 +31,14 @@ struct WorkPolicy {
     }
 
     // whether a workspace of `now` bytes goes back to the device after a call that could have run in `need` bytes and
-    // began with a workspace of `before`
-    static bool give_back(size_t now, size_t before, size_t need) { return now > std::max(before, need) + kWorkKeep; }
+    // began with a workspace of `before`; below a limit of the caller's nothing does
+    bool give_back(size_t now, size_t before, size_t need) const
+    {
+        return !limit && now > std::max(before, need) + kWorkKeep;
+    }
 
     // the most a call takes for speed alone, with a workspace of `have` bytes there already
-    static size_t budget(size_t have) { return std::max(have, kWorkKeep); }
+    size_t budget(size_t have) const { return std::max(have, limit ? limit : kWorkKeep); }
 };
 
 }  // namespace kq

@@ -70,6 +70,7 @@ EXPORTED_SYMBOLS = [
     "kq_slab_cgm_state_bytes", "kq_slab_cgm_init", "kq_slab_cgm_step",
     "kq_slab_cgm_residual", "kq_slab_cgm_update", "kq_slab_cgm_poll", "kq_host_alloc", "kq_host_free", "kq_apply_host",
     "kq_vec_axpby", "kq_vec_dot",
+    "kq_set_workspace_limit",
     "kq_solve_multishift", "kq_solve_multishift_device", "kq_true_residuals", "kq_make_links_record",
     "kq_make_source_record", "kq_last_error", "kq_batch_create", "kq_batch_destroy", "kq_batch_add",
     "kq_batch_size", "kq_batch_solve", "kq_batch_system_info", "kq_net_create", "kq_net_destroy",
@@ -118,6 +119,7 @@ def library() -> C.CDLL:
         "kq_context_destroy": (None, [vp]),
         "kq_load_links": (i, [vp, i, vp, i]),
         "kq_prepare_links": (i, [vp, i]),
+        "kq_set_workspace_limit": (i, [vp, sz]),
         "kq_spinor_bytes": (sz, [vp, i]),
         "kq_spinor_upload": (i, [vp, i, vp, i, vp, vp]),
         "kq_spinor_download": (i, [vp, i, vp, vp, i, vp]),
@@ -379,6 +381,10 @@ class Context:
         self._chk(library().kq_solve_multishift_device(self._h, C.byref(p), _ptr(d_b), _ptr(d_x), C.byref(info)),
                   "kq_solve_multishift_device")
         return info
+
+    def set_workspace_limit(self, nbytes: int):
+        """Keep the device workspace within nbytes where a call can do with less (0: the library's own rule)."""
+        self._chk(library().kq_set_workspace_limit(self._h, int(nbytes)), "kq_set_workspace_limit")
 
     def true_residuals(self, parity, sigmas, d_b, d_x):
         sg = (C.c_double * len(sigmas))(*[float(s) for s in sigmas])

@@ -31,9 +31,14 @@ int main()
     printf("%d %d %d %d\n", p.may_grow(199 * M, 0, 900 * M, 4), p.may_grow(200 * M, 0, 900 * M, 4),
            p.may_grow(220 * M, 50 * M, 850 * M, 4), p.may_grow(200 * M, 0, 901 * M, 4));
     // what goes back: more than 512 MiB above what the call needed and found
-    printf("%d %d %d\n", WorkPolicy::give_back(612 * M, 0, 100 * M), WorkPolicy::give_back(612 * M + 1, 0, 100 * M),
-           WorkPolicy::give_back(612 * M + 1, 612 * M + 1, 100 * M));
-    printf("%d %d\n", (int)(WorkPolicy::budget(0) / M), (int)(WorkPolicy::budget(700 * M) / M));
+    printf("%d %d %d\n", p.give_back(612 * M, 0, 100 * M), p.give_back(612 * M + 1, 0, 100 * M),
+           p.give_back(612 * M + 1, 612 * M + 1, 100 * M));
+    printf("%d %d\n", (int)(p.budget(0) / M), (int)(p.budget(700 * M) / M));
+    // a limit of the caller's takes the place of the 512 MiB, and nothing below it goes back
+    WorkPolicy q;
+    q.limit = 64 * M;
+    printf("%d %d %d %d %d\n", q.may_grow(64 * M, 0, 800 * M, 4), q.may_grow(65 * M, 0, 800 * M, 4),
+           q.give_back(612 * M + 1, 0, 0), (int)(q.budget(0) / M), (int)(q.budget(700 * M) / M));
 }
 """
 
@@ -43,7 +48,7 @@ def test_policy(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-I", str(ROOT / "kuqcd_b200" / "csrc"), str(tmp_path / "w.cpp"), "-o",
                     str(tmp_path / "w")], check=True)
     out = subprocess.run([str(tmp_path / "w")], check=True, capture_output=True, text=True).stdout.splitlines()
-    assert out == ["1 0 1 1", "1 0 0 1", "0 1 0", "512 700"]
+    assert out == ["1 0 1 1", "1 0 0 1", "0 1 0", "512 700", "1 0 0 64 700"]
 
 
 def held(before):
