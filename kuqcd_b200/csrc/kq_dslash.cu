@@ -100,14 +100,18 @@ __global__ void __launch_bounds__(S *split_sites(S)) dslash_split_kernel(Geom g,
 // HALF kernel: 0 one site per thread, 4 .. 7 two sites per thread in packed FP32 with 4 .. 7 resident 128-thread
 // CTAs per SM (KUQCD_HALF_DSLASH = site | pair4 | pair5 | pair6 | pair7).  Default pair7: the kernel is latency-
 // bound, and 28 warps per SM at 72 registers (40 B of spills) beat 20 at 96 (48^3x96: 536 against 577 us).
-static int half_kernel()
+// A kernel named there runs at every size; without one the size decides (launch_dslash2).
+struct HalfKernel {
+    int ctas;
+    bool named;
+};
+static const HalfKernel &half_kernel()
 {
-    static const int k = [] {
+    static const HalfKernel k = []() -> HalfKernel {
         const char *e = getenv("KUQCD_HALF_DSLASH");
-        if (!e) return 7;
-        if (e[0] == 's') return 0;
-        if (strncmp(e, "pair", 4) == 0 && e[4] >= '4' && e[4] <= '7' && e[5] == 0) return e[4] - '0';
-        return 7;
+        if (e && e[0] == 's') return {0, true};
+        if (e && strncmp(e, "pair", 4) == 0 && e[4] >= '4' && e[4] <= '7' && e[5] == 0) return {e[4] - '0', true};
+        return {7, false};
     }();
     return k;
 }
@@ -125,6 +129,7 @@ static bool pair_ok(int lp, int sp)
 
 static int threads_per_site(int lp, int sites)
 {
+    if (lp == P16 && half_kernel().named) return 1;
     return split_of(sites, lp == P64 ? kSplitLimit64 : lp == P32 ? kSplitLimit32 : kSplitLimit16);
 }
 
@@ -173,10 +178,10 @@ cudaError_t launch_dslash2(const Geom &g, const GaugeDev &gd, int lp, int sp, co
     const int pv = pad_sites(g.vh);
     // HALF: two sites per thread in packed FP32 (kq_dslash_half2.cuh) on lattices of some waves of it; below, one site
     // per thread is ahead (80,000 sites 12.6 against 13.2 us, 165,888 21.7 against 21.6 us)
-    if (lp == P16 && sp == P16 && !gate && half_kernel() != 0 && g.vh > 150000) {
+    if (lp == P16 && sp == P16 && !gate && half_kernel().ctas != 0 && (half_kernel().named || g.vh > 150000)) {
         constexpr int kBS2 = 128;
         const int nb2 = (g.vh + 2 * kBS2 - 1) / (2 * kBS2);
-        switch (half_kernel()) {
+        switch (half_kernel().ctas) {
             case 4: dslash_half2_kernel<kBS2, 4><<<nb2, kBS2, 0, s>>>(g, pv, gd.fat[lp], gd.lng[lp], src, dst, dst_parity); break;
             case 6: dslash_half2_kernel<kBS2, 6><<<nb2, kBS2, 0, s>>>(g, pv, gd.fat[lp], gd.lng[lp], src, dst, dst_parity); break;
             case 7: dslash_half2_kernel<kBS2, 7><<<nb2, kBS2, 0, s>>>(g, pv, gd.fat[lp], gd.lng[lp], src, dst, dst_parity); break;
