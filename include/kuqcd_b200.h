@@ -265,7 +265,8 @@ typedef struct kq_batch kq_batch;
 typedef struct {
     int num_systems;
     int iterations;           /* largest iteration count over the systems */
-    double batched_seconds;   /* device time of the batched iterations */
+    double batched_seconds;   /* time on the stream from the first batched iteration to the last, with the launches and
+                                 polls between chunks */
     long long kernel_launches;
     int tile;                 /* sites per tile = threads per CTA */
     int ctas_per_sm;          /* persistent grid: CTAs per SM */
