@@ -391,8 +391,8 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
     long long launches = 1;
 
     // One graph per operator precision, each kChunk iterations + the window update.  Building one takes the host about
-    // 130 us (and its first launch more): the first two chunks are enqueued kernel by kernel and the graphs built while
-    // they run.
+    // 130 us (and its first launch more): the first chunk is enqueued kernel by kernel and the graphs built while it
+    // runs.
     cudaGraphExec_t *exec = res->exec;
     char *host_poll = reinterpret_cast<char *>(ctx->poll);
     auto build = [&](int m) -> cudaError_t {
@@ -410,7 +410,8 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
     // that the GPU does not idle through a poll and a graph launch after every kChunk iterations (35 us of a chunk's
     // 170 us at 8^4).  The next chunk is launched ahead only where the last two states predict that the one in flight
     // neither ends the solve nor reaches a switch of precision; a wrong guess costs a chunk of no-ops, or keeps the
-    // higher precision for kChunk more iterations.  The guess depends on the iterates alone, so a solve repeats
+    // higher precision for kChunk more iterations.  Nothing is launched ahead of the first state, which is all that a
+    // short solve has (two iterations at 4^4: 330 us, with a second chunk ahead 430 us).  The guess depends on the iterates alone, so a solve repeats
     // exactly.
     cudaEvent_t done[2] = {nullptr, nullptr};
     cudaError_t err = cudaSuccess;
@@ -442,15 +443,17 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
         final_from = std::min(final_from, mt);
     };
     const int most = max_iter / kChunk + 3;  // chunks: every solve has stopped by then while its state is consistent
-    double rel2 = 1.0, fall = 1e-2;  // |r|^2 / |b|^2 of the last state read, and its factor over the chunk before it
+    double rel2 = 1.0, fall = 1.0;  // |r|^2 / |b|^2 of the last state read, and its factor over the chunk before it
     double stop2 = 0.0;              // the tolerance in the same units, once |b|^2 is known
     launch(mode_of(rel2));
     while (err == cudaSuccess) {
         const int m = mode_of(rel2);
         const double guess = rel2 * std::min(fall, 1.0);  // state after the chunk in flight
-        if (launched < most && guess > stop2 && mode_of(0.1 * guess) == m) launch(m);
+        // (a chunk runs kChunk iterations unless it ends the solve, so the cap says when the last one has been launched)
+        const auto more = [&] { return launched < most && (long long)launched * kChunk < max_iter; };
+        if (polled > 0 && more() && guess > stop2 && mode_of(0.1 * guess) == m) launch(m);
         // a graph that will be wanted, one per chunk in flight
-        for (int b : {m, use32 ? 1 : 0, use16 ? 2 : 0})
+        if (more()) for (int b : {m, use32 ? 1 : 0, use16 ? 2 : 0})
             if (err == cudaSuccess && !exec[b] && b >= m) {
                 err = build(b);
                 break;
