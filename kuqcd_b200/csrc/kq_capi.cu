@@ -63,8 +63,9 @@ bool optional_work(::kq_context *ctx, size_t want, int share)
 {
     if (ctx->work_bytes >= want) return true;
     const size_t have = ctx->work_bytes;
-    size_t free = 0, total = 0;
-    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    const bool asked = ctx->work_policy.asks(want, have);
+    size_t free = ~size_t(0) >> 1, total = 0;
+    if (asked && cudaMemGetInfo(&free, &total) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -73,7 +74,12 @@ bool optional_work(::kq_context *ctx, size_t want, int share)
     if (ensure_work(ctx, want) == cudaSuccess) return true;
     cudaGetLastError();
     set_last_error(text);
-    ctx->work_policy.note_failure(want, have, free);
+    // the old workspace is gone: what is free now is the room there was
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+        cudaGetLastError();
+        free = 0;
+    }
+    ctx->work_policy.note_failure(want, free);
     return false;
 }
 

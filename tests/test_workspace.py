@@ -27,9 +27,12 @@ int main()
     printf("%d %d %d %d\n", p.may_grow(300 * M, 100 * M, 800 * M, 4), p.may_grow(301 * M, 100 * M, 800 * M, 4),
            p.may_grow(301 * M, 100 * M, 800 * M, 1), p.may_grow(100 * M, 100 * M, 0, 4));
     // a failure at 200 MiB with room for 900: no second try at that size or above until there is more room
-    p.note_failure(200 * M, 100 * M, 800 * M);
+    p.note_failure(200 * M, 900 * M);
     printf("%d %d %d %d\n", p.may_grow(199 * M, 0, 900 * M, 4), p.may_grow(200 * M, 0, 900 * M, 4),
            p.may_grow(220 * M, 50 * M, 850 * M, 4), p.may_grow(200 * M, 0, 901 * M, 4));
+    // the free memory is looked at for more than 64 MiB, and for anything after a failure
+    printf("%d %d %d %d\n", WorkPolicy().asks(164 * M, 100 * M), WorkPolicy().asks(164 * M + 1, 100 * M),
+           WorkPolicy().asks(M, 100 * M), p.asks(M, 0));
     // what goes back: more than 512 MiB above what the call needed and found
     printf("%d %d %d\n", p.give_back(612 * M, 0, 100 * M), p.give_back(612 * M + 1, 0, 100 * M),
            p.give_back(612 * M + 1, 612 * M + 1, 100 * M));
@@ -48,7 +51,7 @@ def test_policy(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-I", str(ROOT / "kuqcd_b200" / "csrc"), str(tmp_path / "w.cpp"), "-o",
                     str(tmp_path / "w")], check=True)
     out = subprocess.run([str(tmp_path / "w")], check=True, capture_output=True, text=True).stdout.splitlines()
-    assert out == ["1 0 1 1", "1 0 0 1", "0 1 0", "512 700", "1 0 0 64 700"]
+    assert out == ["1 0 1 1", "1 0 0 1", "0 1 0 1", "0 1 0", "512 700", "1 0 0 64 700"]
 
 
 def held(before):
