@@ -83,6 +83,30 @@ bool optional_work(::kq_context *ctx, size_t want, int share)
     return false;
 }
 
+void *pool_work(::kq_context *ctx, size_t want, int share)
+{
+    size_t free = 0, total = 0;
+    uint64_t unused = 0;
+    if (!ctx->work_pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = ctx->device;
+        uint64_t keep = ~uint64_t(0);
+        if (cudaMemPoolCreate(&ctx->work_pool, &props) != cudaSuccess) ctx->work_pool = nullptr;
+        else cudaMemPoolSetAttribute(ctx->work_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    void *p = nullptr;
+    if (ctx->work_pool && cudaMemPoolGetAttribute(ctx->work_pool, cudaMemPoolAttrReservedMemCurrent, &unused) == cudaSuccess &&
+        cudaMemGetInfo(&free, &total) == cudaSuccess && ctx->work_policy.may_grow(want, 0, free + unused, share) &&
+        cudaMallocFromPoolAsync(&p, want, ctx->work_pool, ctx->stream) != cudaSuccess) {
+        ctx->work_policy.note_failure(want, free + unused);
+        p = nullptr;
+    }
+    cudaGetLastError();  // the caller goes on without it
+    return p;
+}
+
 static cudaError_t alloc_links(::kq_context *ctx, int prec)
 {
     if (ctx->gd.block[prec]) return cudaSuccess;
@@ -177,6 +201,7 @@ KQ_API void kq_context_destroy(kq_context *ctx)
     for (void *gl : ctx->ghost_links)
         if (gl) cudaFree(gl);
     if (ctx->work) cudaFree(ctx->work);
+    if (ctx->work_pool) cudaMemPoolDestroy(ctx->work_pool);
     if (ctx->io) cudaFree(ctx->io);
     if (ctx->d_scratch) cudaFree(ctx->d_scratch);
     if (ctx->poll) cudaFreeHost(ctx->poll);
@@ -303,13 +328,11 @@ KQ_API KuQCDStatus kq_set_workspace_limit(kq_context *ctx, size_t bytes)
 {
     if (!ctx) return KUQCD_ERR_NULL_POINTER;
     ctx->work_policy.limit = bytes;
-    if (bytes && ctx->work_bytes > bytes) {
-        cudaSetDevice(ctx->device);
-        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
-        release_work(ctx);
-        return status_of(e);
-    }
-    return KUQCD_SUCCESS;
+    cudaSetDevice(ctx->device);
+    cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    if (bytes && ctx->work_bytes > bytes) release_work(ctx);
+    if (e == cudaSuccess && ctx->work_pool) e = cudaMemPoolTrimTo(ctx->work_pool, 0);
+    return status_of(e);
 }
 
 KQ_API size_t kq_spinor_bytes(const kq_context *ctx, int prec)
@@ -523,14 +546,17 @@ KQ_API KuQCDStatus kq_true_residuals(kq_context *ctx, int parity, int num_shift,
 static KuQCDStatus solve_full(kq_context *ctx, const kq_solve_param *p, const void *d_b, void *d_x,
                               kq_solve_info *info);
 
-// multishift CG with windowed shift updates, all in FP64 (kq_msrelax.cu)
+// multishift CG with windowed shift updates, all in FP64 (kq_msrelax.cu), in `work` (null: the context's workspace)
 static cudaError_t windowed_solve(kq_context *ctx, const kq_solve_param *p, const double *sig, const void *d_b,
-                                  void *d_x, kq_solve_info *info)
+                                  void *d_x, kq_solve_info *info, void *work = nullptr)
 {
     MsBuffers w;
-    const cudaError_t e = ensure_work(ctx, ms_workspace_bytes(ctx->g, p->num_shift));
-    if (e != cudaSuccess) return e;
-    Carve c(ctx->work);
+    if (!work) {
+        const cudaError_t e = ensure_work(ctx, ms_workspace_bytes(ctx->g, p->num_shift));
+        if (e != cudaSuccess) return e;
+        work = ctx->work;
+    }
+    Carve c(work);
     ms_layout(c, ctx->g, p->num_shift, d_b, d_x, w);
     double rs[kMaxShift];
     rs[0] = sig[0];
@@ -559,8 +585,6 @@ KQ_API KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_pa
     memset(info, 0, sizeof(*info));
     info->num_shift = p->num_shift;
 
-    const size_t work_before = ctx->work_bytes;
-    size_t work_need = 0;  // what the call can do with, where that is less than what it takes
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -583,8 +607,8 @@ KQ_API KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_pa
         // In FP64 the windowed solver takes the same steps with (4 N + 16) / 16 instead of 4 N vector passes per
         // iteration for N shifts and three kernels instead of four: 24^3 x 48, 12 shifts, 0.303 ms per iteration in
         // the reference's kernel order and 0.235 ms windowed.  It takes a ring of 16 residuals; where that is more
-        // than a quarter of the device's free memory or than the caller's limit, and in FP32 (whose recurrences would lose digits in the
-        // window's products), the reference's kernel order remains.
+        // than a quarter of the device's free memory or than the caller's limit, and in FP32 (whose recurrences would
+        // lose digits in the window's products), the reference's kernel order remains.
         const Geom &g = ctx->g;
         const size_t vb = spinor_bytes(g, prec), vb64 = spinor_bytes(g, P64);
         const int nb = (g.vh + 255) / 256;
@@ -608,18 +632,20 @@ KQ_API KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_pa
         CgmBuffers w;
         Carve probe(nullptr);
         layout(probe, w);
-        // Where the workspace for it goes back after the call (kq_work.h), allocating and freeing it takes 1.4 ms at
-        // 700 MB (8 ms at 8 GB), which short solves do not earn: 0.03 ms per iteration with one shift, 0.27 ms with
-        // twelve at 40 x 40 x 32 x 32.
+        // A workspace that may not stay with the context comes from its pool.  Mapping it for the first time takes
+        // 6 ms per GB, which short solves do not earn (0.03 ms per iteration with one shift, 0.27 ms with twelve at
+        // 40 x 40 x 32 x 32); allocating and freeing it in every call took up to 0.47 s of a 3.9 s solve at 48^3 x 96.
         const size_t want = ms_workspace_bytes(g, ns);
-        const bool pays = !ctx->work_policy.give_back(want, ctx->work_bytes, probe.off) || p->max_iter >= 64;
-        if (prec == P64 && pays && optional_work(ctx, want, 4)) {
-            work_need = probe.off;
+        const bool keeps = ctx->work_policy.keeps(want, ctx->work_bytes, probe.off);
+        void *pooled = nullptr;
+        if (prec == P64 && !keeps && p->max_iter >= 64) pooled = pool_work(ctx, want, 4);
+        if (pooled || (prec == P64 && keeps && optional_work(ctx, want, 4))) {
             // this solver reports no solution before its end
             auto *const ready = ctx->solution_ready;
             ctx->solution_ready = nullptr;
-            e = windowed_solve(ctx, p, sig, d_b, d_x, info);
+            e = windowed_solve(ctx, p, sig, d_b, d_x, info, pooled);
             ctx->solution_ready = ready;
+            if (pooled) cudaFreeAsync(pooled, ctx->stream);
             if (e == cudaSuccess && info->status == 0 && info->iter >= p->max_iter) info->status = KQ_STATUS_MAXITER;
         } else {
             e = ensure_work(ctx, probe.off);
@@ -652,10 +678,6 @@ KQ_API KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_pa
     info->seconds = ms * 1e-3;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (work_need && ctx->work_policy.give_back(ctx->work_bytes, work_before, work_need)) {
-        cudaStreamSynchronize(ctx->stream);
-        release_work(ctx);
-    }
     if (e != cudaSuccess) {
         if (std::string(last_error()).empty()) set_last_error(cudaGetErrorString(e));
         return status_of(e);

@@ -17,6 +17,7 @@ struct kq_context {
     void *work = nullptr;
     size_t work_bytes = 0;
     kq::WorkPolicy work_policy;
+    cudaMemPool_t work_pool = nullptr;  // larger workspaces, for the duration of one call (created on first use)
     // device fields and host-record staging of kq_solve_multishift (host buffers in and out), grown on demand
     void *io = nullptr;
     size_t io_bytes = 0;
@@ -59,6 +60,8 @@ cudaError_t ensure_work(::kq_context *ctx, size_t bytes);
 // this is false goes on in less (last error and its text are as before)
 bool optional_work(::kq_context *ctx, size_t want, int share);
 void release_work(::kq_context *ctx);
+// `want` bytes from the context's pool under its policy, or null; given back in stream order with cudaFreeAsync
+void *pool_work(::kq_context *ctx, size_t want, int share);
 KuQCDStatus status_of(cudaError_t e);
 
 // KQ_SOLVER_MIXED on one context (kq_mixed.cu); shifts_abs are absolute.  With run_phase1 = false, d_x already

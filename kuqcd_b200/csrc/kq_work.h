@@ -7,8 +7,9 @@ namespace kq {
 
 // Workspace that calls keep for speed alone.  512 MiB is 0.3 % of a B200's memory and holds all that the solver and the
 // residual check ask for up to 32^4 with 12 shifts (378 MB more for the windowed solver, 302 MB of temporaries).
-// Beyond it a solve takes its workspace anew, 3.6 of 604 ms at 48^4, and a residual check in a context that has solved
-// nothing takes fewer shifts at a time, 9.0 against 8.3 ms there.
+// Beyond it a solve's workspace comes from the context's pool, whose memory the driver hands to any allocation of the
+// process that would fail without it, and a residual check in a context that has solved nothing takes fewer shifts at a
+// time (48^4, 12 shifts: 9.0 against 8.3 ms).
 constexpr size_t kWorkKeep = size_t(512) << 20;
 
 // Growth that is taken without a look at the free memory, which costs the host 70 us: 64 MiB, unless an allocation has
@@ -38,12 +39,9 @@ struct WorkPolicy {
         failed_room = room;
     }
 
-    // whether a workspace of `now` bytes goes back to the device after a call that could have run in `need` bytes and
-    // began with a workspace of `before`; below a limit of the caller's nothing does
-    bool give_back(size_t now, size_t before, size_t need) const
-    {
-        return !limit && now > std::max(before, need) + kWorkKeep;
-    }
+    // whether a call that could run in `need` bytes may leave a workspace of `want` behind, `have` bytes being there; a
+    // limit of the caller's takes the place of the rule
+    bool keeps(size_t want, size_t have, size_t need) const { return limit || want <= std::max(have, need) + kWorkKeep; }
 
     // the most a call takes for speed alone, with a workspace of `have` bytes there already
     size_t budget(size_t have) const { return std::max(have, limit ? limit : kWorkKeep); }

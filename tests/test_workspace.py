@@ -33,15 +33,15 @@ int main()
     // the free memory is looked at for more than 64 MiB, and for anything after a failure
     printf("%d %d %d %d\n", WorkPolicy().asks(164 * M, 100 * M), WorkPolicy().asks(164 * M + 1, 100 * M),
            WorkPolicy().asks(M, 100 * M), p.asks(M, 0));
-    // what goes back: more than 512 MiB above what the call needed and found
-    printf("%d %d %d\n", p.give_back(612 * M, 0, 100 * M), p.give_back(612 * M + 1, 0, 100 * M),
-           p.give_back(612 * M + 1, 612 * M + 1, 100 * M));
+    // what stays with the context: up to 512 MiB above what the call needs or found
+    printf("%d %d %d\n", p.keeps(612 * M, 0, 100 * M), p.keeps(612 * M + 1, 0, 100 * M),
+           p.keeps(612 * M + 1, 612 * M + 1, 100 * M));
     printf("%d %d\n", (int)(p.budget(0) / M), (int)(p.budget(700 * M) / M));
-    // a limit of the caller's takes the place of the 512 MiB, and nothing below it goes back
+    // a limit of the caller's takes the place of the 512 MiB
     WorkPolicy q;
     q.limit = 64 * M;
     printf("%d %d %d %d %d\n", q.may_grow(64 * M, 0, 800 * M, 4), q.may_grow(65 * M, 0, 800 * M, 4),
-           q.give_back(612 * M + 1, 0, 0), (int)(q.budget(0) / M), (int)(q.budget(700 * M) / M));
+           q.keeps(612 * M + 1, 0, 0), (int)(q.budget(0) / M), (int)(q.budget(700 * M) / M));
 }
 """
 
@@ -51,7 +51,7 @@ def test_policy(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-I", str(ROOT / "kuqcd_b200" / "csrc"), str(tmp_path / "w.cpp"), "-o",
                     str(tmp_path / "w")], check=True)
     out = subprocess.run([str(tmp_path / "w")], check=True, capture_output=True, text=True).stdout.splitlines()
-    assert out == ["1 0 1 1", "1 0 0 1", "0 1 0 1", "0 1 0", "512 700", "1 0 0 64 700"]
+    assert out == ["1 0 1 1", "1 0 0 1", "0 1 0 1", "1 0 1", "512 700", "1 0 1 64 700"]
 
 
 def held(before):
@@ -62,33 +62,43 @@ def held(before):
 @pytest.mark.gpu
 def test_memory_left_behind_by_solves_and_checks(cuda):
     """At 48 x 48 x 32 x 32 an FP64 field is 54 MiB: the windowed FP64 solve of 12 shifts works in 30 of them where the
-    reference's kernel order needs 15, and the residual check would take 12.  What stays is at most 512 MiB above what
-    the calls cannot do without (64 MiB of slack for the kernels' code and the partial sums)."""
+    reference's kernel order needs 15, and the residual check would take 12.  What later allocations of the process cannot
+    have is at most 512 MiB above what the calls cannot do without (64 MiB of slack for the kernels' code and the partial
+    sums): one allocation of all the rest succeeds, and the next solve works."""
     dims, ns, slack = (48, 48, 32, 32), 12, 64 * MIB
     v = int(np.prod(dims))
     ctx = K.Context(dims)
-    rec = np.full(v * 72, 0.1)
+    rng = np.random.default_rng(1)
+    rec = 0.1 * rng.standard_normal(v * 72)
     ctx.load_links(K.KUQCD_FAT_LINK, rec)
     ctx.load_links(K.KUQCD_LONG_LINK, rec)
+    del rec
     vb = ctx.spinor_bytes(K.KUQCD_DOUBLE)
     assert 15 * vb > KEEP + slack
     d_b, d_x = dev_buffer(vb), dev_buffer(ns * vb)
-    ctx.upload(K.KUQCD_DOUBLE, np.random.default_rng(1).standard_normal(v // 2 * 6), d_b)
+    ctx.upload(K.KUQCD_DOUBLE, rng.standard_normal(v // 2 * 6), d_b)
     sig = list(0.01 + np.logspace(-2, 0, ns))
-    kw = dict(tol=0.0, max_iter=3)
     torch.cuda.empty_cache()
     free = torch.cuda.mem_get_info()[0]
     first = ctx.true_residuals(0, sig, d_b, d_x)
     assert held(free) <= KEEP + slack
-    for _ in range(2):  # a second solve finds what the first left
-        ctx.solve_device(d_b, d_x, sig, solver=K.KQ_SOLVER_CGM, **kw)
-        assert held(free) <= (ns + 3) * vb + KEEP + slack
     assert np.allclose(first, 1.0, rtol=1e-12, atol=0)  # x = 0
+    solutions = []
+    for cap in (64, 64, 3):  # windowed, windowed with what the first left, in the reference's order
+        info = ctx.solve_device(d_b, d_x, sig, solver=K.KQ_SOLVER_CGM, tol=0.0, max_iter=cap)
+        assert info.kernel_launches == (1 + 32 if cap == 3 else 1 + 8 * 26)
+        solutions.append(d_x.cpu())
+        rest = torch.empty(free - (ns + 3) * vb - KEEP - slack, dtype=torch.uint8, device="cuda")
+        del rest
+        torch.cuda.empty_cache()
+    assert torch.equal(solutions[0], solutions[1])
     # the explicit windowed solver needs its ring and keeps it; the others then use what is there
-    ctx.solve_device(d_b, d_x, sig, solver=K.KQ_SOLVER_CGM_WINDOWED, **kw)
+    ctx.solve_device(d_b, d_x, sig, solver=K.KQ_SOLVER_CGM_WINDOWED, tol=0.0, max_iter=64)
+    assert torch.equal(solutions[0], d_x.cpu())
+    ctx.set_workspace_limit(0)
     ring = held(free)
     assert ring >= (ns + 18) * vb
     ctx.true_residuals(0, sig, d_b, d_x)
-    ctx.solve_device(d_b, d_x, sig, solver=K.KQ_SOLVER_CGM, **kw)
+    ctx.solve_device(d_b, d_x, sig, solver=K.KQ_SOLVER_CGM, tol=0.0, max_iter=64)
     assert abs(held(free) - ring) <= slack
     ctx.close()
