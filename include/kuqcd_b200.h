@@ -243,11 +243,12 @@ KuQCDStatus kq_solve_multishift(kq_context *ctx, const kq_solve_param *param, co
  * that for KQ_PARITY_FULL). */
 KuQCDStatus kq_solve_multishift_device(kq_context *ctx, const kq_solve_param *param, const void *d_b, void *d_x,
                                        kq_solve_info *info);
-/* The most bytes of workspace this context holds on the device where a call can do with less; a larger workspace held
- * from earlier calls is freed.  0 (the default): calls take at most a quarter of the free memory for speed alone and
- * keep at most 512 MiB of it.  What depends on it: KQ_SOLVER_CGM in FP64 (num_shift + 18 FP64 fields, or num_shift + 3
- * in the reference's kernel order, 0.303 against 0.235 ms per iteration at 24^3 x 48 with 12 shifts) and
- * kq_true_residuals (one field of one parity for each of up to 16 shifts at a time; without a limit at least two). */
+/* The most bytes of workspace this context holds on the device where a call can do with less; what is held above that
+ * from earlier calls is freed.  0 (the default): calls take at most a quarter of the free memory for speed alone, keep
+ * at most 512 MiB of it, and leave the rest where any allocation of the process can have it.  What depends on it:
+ * KQ_SOLVER_CGM in FP64 (num_shift + 18 FP64 fields, or num_shift + 3 in the reference's kernel order, 0.303 against
+ * 0.235 ms per iteration at 24^3 x 48 with 12 shifts) and kq_true_residuals (one field of one parity for each of up to
+ * 16 shifts at a time; without a limit at least two). */
 KuQCDStatus kq_set_workspace_limit(kq_context *ctx, size_t bytes);
 /* FP64 true relative residuals |b - (sigma_k - DD) x_k| / |b| of device FP64 fields (absolute sigmas; parity
  * KQ_PARITY_FULL: full-lattice fields, norms over both parities). */

@@ -1,6 +1,6 @@
 // Multishift CG (CGM) on the device with the reference's recurrences, stopping rule and kernel order
-// (inverter_cgm.cpp:17-87).  FP32 solves run here, and FP64 ones where the device has no room for the residual ring of
-// the windowed solver (kq_msrelax.cu), which is a quarter faster:
+// (inverter_cgm.cpp:17-87).  FP32 solves run here, and FP64 ones that may not have the workspace of the windowed solver
+// (kq_msrelax.cu; kq_set_workspace_limit), which is a quarter faster:
 //   x_0 solves (shifts[0] - D_pq D_qp) x = b,  x_j (j >= 1) solves (shifts[0] + shifts[j] - D_pq D_qp) x = b;
 //   shift k stops when Z_k^2 |r|^2 < tol, dropped from the end of the list; iteration ends when no shift is left or
 //   iter reaches max_iter.

@@ -231,7 +231,9 @@ __host__ __device__ constexpr int split_sites(int S) { return S == 2 ? 64 : 32; 
 // wave of the kernel (FP64 113,664 threads, FP32 189,440).  Beyond it the extra CTAs only add partial sums.  Measured
 // with S = 1 / 2 / 4 / 8 (us): FP64 12,096 sites 9.7 / 6.4 / 4.8 / 4.5, 24,192 10.8 / 7.7 / 8.7 / 7.9, 41,472 17.2 / 11.5
 // / 12.9 / 14.9, 52,488 20.0 / 22.3; FP32 24,192 8.4 / 5.8 / 4.7 / 5.0, 41,472 9.1 / 6.6 / 6.3 / 6.8, 80,000 15.0 / 11.0,
-// 120,000 20.6 / 22.8; HALF 19,208 6.3 / 5.4 / 4.7 / 5.1, 41,472 9.0 / 7.3 / 7.0 / 7.6, 65,536 9.2 / 9.4.
+// 120,000 20.6 / 22.8; HALF 19,208 6.3 / 5.4 / 4.7 / 5.1, 41,472 9.0 / 7.3 / 7.0 / 7.6, 65,536 9.2 / 9.4.  One limit per
+// precision gives up 0.3 us at two of these sizes (FP64 12,096 and HALF 41,472 would run 0.3 us faster with twice the
+// threads that the rule takes).
 constexpr int kSplitLimit64 = 94000, kSplitLimit32 = 175000, kSplitLimit16 = 150000;
 inline int split_of(int sites, int limit)
 {

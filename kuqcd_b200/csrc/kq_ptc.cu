@@ -254,9 +254,10 @@ __global__ void __launch_bounds__(kThr) ptc_forward_kernel(Geom g, int pv, LinkS
 // tensor cores multiply chunk j - 1 from the other, so shared memory holds 2 x 3 x [128 x 16] BF16 (24 KB) instead
 // of the whole [128 x 144] tile per colour (108 KB).  Chunk j's MMAs commit to mbarrier (j & 1); before chunk j + 2
 // overwrites that buffer every thread waits for the commit's phase (j >> 1) & 1 (bounded, as in the whole-tile kernel).
-// The layer is bound by the latency of the gather, 24 scattered 8-byte loads per site and path: the loads of path j + 1
-// are issued once path j's values are used, ahead of its barriers.  32^4, 8 -> 8 channels: 356 us with four CTAs per SM
-// at 128 registers; without the early loads 450 us with six at 80.  One application of M: 1.23 ms (1.50 ms before); with
+// The gather is 24 scattered 8-byte loads per site and path: the loads of path j + 1 are issued once path j's values are
+// used, ahead of its barriers.  32^4, 8 -> 8 channels: 356 us with four CTAs per SM at 128 registers; without the early
+// loads 450 us with six at 80, most of it spent waiting for them (long scoreboard 3.9 stalled warps per issue; now 0.5,
+// with 68 % of the issue slots used, DRAM at 25 %).  One application of M: 1.23 ms (1.50 ms before); with
 // two or four threads per site, each loading the links again, 1.38 and 1.78 ms; with the next loads issued channel by
 // channel among the mat-vecs 1.43 ms.
 constexpr uint32_t kChunkColBytes = kTile * 16 * 2;  // one colour's [128 x 16] BF16 chunk
