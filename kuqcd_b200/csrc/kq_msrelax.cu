@@ -391,8 +391,8 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
     long long launches = 1;
 
     // One graph per operator precision, each kChunk iterations + the window update.  Building one takes the host about
-    // 130 us (and its first launch more): the first chunk is enqueued kernel by kernel and the graphs built while it
-    // runs.
+    // 130 us (and its first launch more): the first three chunks are enqueued kernel by kernel and the graphs built
+    // once two of them are in flight, so that a solve of one chunk builds none.
     cudaGraphExec_t *exec = res->exec;
     char *host_poll = reinterpret_cast<char *>(ctx->poll);
     auto build = [&](int m) -> cudaError_t {
@@ -411,8 +411,8 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
     // 170 us at 8^4).  The next chunk is launched ahead only where the last two states predict that the one in flight
     // neither ends the solve nor reaches a switch of precision; a wrong guess costs a chunk of no-ops, or keeps the
     // higher precision for kChunk more iterations.  Nothing is launched ahead of the first state, which is all that a
-    // short solve has (two iterations at 4^4: 330 us, with a second chunk ahead 430 us).  The guess depends on the iterates alone, so a solve repeats
-    // exactly.
+    // short solve has (two iterations at 4^4: 130 us; with a second chunk ahead and a graph built beside the first
+    // 430 us).  The guess depends on the iterates alone, so a solve repeats exactly.
     cudaEvent_t done[2] = {nullptr, nullptr};
     cudaError_t err = cudaSuccess;
     for (auto &ev : done)
@@ -421,7 +421,7 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
     int launched = 0, polled = 0;
     auto mode_of = [&](double rel2) { return use16 && rel2 < rho16 * rho16 ? 2 : use32 && rel2 < rho32 * rho32 ? 1 : 0; };
     auto launch = [&](int m) {
-        if (err == cudaSuccess && launched >= 2 && !exec[m]) err = build(m);
+        if (err == cudaSuccess && launched >= 3 && !exec[m]) err = build(m);
         if (err == cudaSuccess) {
             if (exec[m]) err = cudaGraphLaunch(exec[m], s);
             else {
@@ -453,11 +453,12 @@ cudaError_t ms_solve(::kq_context *ctx, const MsBuffers &w, int parity, int ns, 
         const auto more = [&] { return launched < most && (long long)launched * kChunk < max_iter; };
         if (polled > 0 && more() && guess > stop2 && mode_of(0.1 * guess) == m) launch(m);
         // a graph that will be wanted, one per chunk in flight
-        if (more()) for (int b : {m, use32 ? 1 : 0, use16 ? 2 : 0})
-            if (err == cudaSuccess && !exec[b] && b >= m) {
-                err = build(b);
-                break;
-            }
+        if (polled > 0 && more())
+            for (int b : {m, use32 ? 1 : 0, use16 ? 2 : 0})
+                if (err == cudaSuccess && !exec[b] && b >= m) {
+                    err = build(b);
+                    break;
+                }
         if (err != cudaSuccess) break;
         err = cudaEventSynchronize(done[polled & 1]);
         if (err != cudaSuccess) break;
