@@ -7,7 +7,7 @@ namespace kq {
 
 // Workspace that calls keep for speed alone.  512 MiB is 0.3 % of a B200's memory and holds all that the solver and the
 // residual check ask for up to 32^4 with 12 shifts (378 MB more for the windowed solver, 302 MB of temporaries).
-// Beyond it a solve's workspace comes from the context's pool, whose memory the driver hands to any allocation of the
+// Beyond it a solve's workspace comes from the context's pool, whose memory CUDA hands to any allocation of the
 // process that would fail without it, and a residual check in a context that has solved nothing takes fewer shifts at a
 // time (48^4, 12 shifts: 9.0 against 8.3 ms).
 constexpr size_t kWorkKeep = size_t(512) << 20;
